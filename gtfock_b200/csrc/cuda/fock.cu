@@ -1,8 +1,8 @@
 // fock.cu -- the PFock engine on one B200.
 //
 // Setup (PFock_create, pfock/pfock.c:801-997):
-//   * device Schwarz screening: one thread per shell pair evaluates the
-//     diagonal quartet (MN|MN) by Rys quadrature and keeps max |(mn|mn)|
+//   * device Schwarz screening (screen.cu): a group of lanes per shell pair
+//     evaluates the diagonal quartet (MN|MN) and keeps max |(mn|mn)|
 //     (pfock/screening.c:59-90); the global max and eta = tol^2/max follow
 //     pfock/screening.c:100,111;
 //   * the reference's CSR pair list (parity rule and signed values,
@@ -37,6 +37,7 @@
 #include "devmem.cuh"
 #include "gtf_cuda.h"
 #include "gtf_dev.cuh"
+#include "sph_dev.cuh"
 // the Fock kernels live in fock_kernel.cuh, instantiated across several
 // translation units (fock_cls_*.cu) so that they compile in parallel
 #include "fock_kernel.cuh"
@@ -97,6 +98,7 @@ struct ClassPairTask {
     int ket_start, nketcls;
     int seg[GTF_NBKT + 1];  // ket segments (primitive-count buckets), relative to ket_start
     long long nunits, nunits32;  // units of the FP64 and the FP32 launch
+    int split_lt;                // lane split of long quartets (gtf_lane_split)
     long long nunits_bound;      // bound on either launch's units under any thresholds >= tol2
     double flops, nprimq;        // Rys-model FLOPs and primitive quartets (before primitive screening)
     double nquart, nquart32;     // quartets in all, of which evaluated in FP32
@@ -288,23 +290,7 @@ static int dalloc(gtf_fock_dev *f, T **p, size_t n)
 
 // ---------------------------------------------------------------------------
 // spherical <-> Cartesian transforms (d shells only)
-// rows m = -2..2, cols xx, xy, xz, yy, yz, zz
 // ---------------------------------------------------------------------------
-__constant__ double c_sph_d[5][6] = {
-    {0.0, 1.7320508075688772, 0.0, 0.0, 0.0, 0.0},
-    {0.0, 0.0, 0.0, 0.0, 1.7320508075688772, 0.0},
-    {-0.5, 0.0, 0.0, -0.5, 0.0, 1.0},
-    {0.0, 0.0, 1.7320508075688772, 0.0, 0.0, 0.0},
-    {0.8660254037844386, 0.0, 0.0, -0.8660254037844386, 0.0, 0.0}};
-
-__device__ __forceinline__ double sph_coef(int L, int pure, int m, int c)
-{
-    if (pure && L == 2) return c_sph_d[m][c];
-    return (m == c) ? 1.0 : 0.0;
-}
-
-__device__ __forceinline__ int nsph_of(int L, int pure) { return (pure && L == 2) ? 5 : ncart(L); }
-
 // D_cart[i][j] = sum_{m,n} T[m][i] T[n][j] D[m][n]
 __device__ __forceinline__ void d_to_cart_elem(const double *__restrict__ D, double *__restrict__ Dc,
                                                const int *__restrict__ cart2shell, const int *__restrict__ sh_L,
@@ -546,102 +532,10 @@ __global__ void k_screen_prep(BasisDev b, const int2 *__restrict__ mn, const int
     make_pair(b, a, bb, off[t], 0, 0, pairs + t, pp, npp);
 }
 
-// Screening slices: the ket components cd = CD0 .. CD0+N-1 (cd = k + NA*l)
-// of the diagonal quartet (MN|MN) at a time, folded into the sums
-// s[m][n] = sum_{i,j,k,l} T[m][i] T[n][j] T[m][k] T[n][l] (ij|kl), so that no
-// thread holds all NA*NB*NA*NB integrals (1296 for (dd|dd)).
-__host__ __device__ constexpr int screen_slice_n(int LA, int LB)
-{
-    // whole quartets up to 81 integrals; else slices of at most 54
-    return ncart(LA) * ncart(LB) * ncart(LA) * ncart(LB) <= 81 ? ncart(LA) * ncart(LB)
-           : ncart(LA) * ncart(LB) * 3 <= 54                   ? 3
-                                                               : 1;
-}
-
-template <int LA, int LB, int CD0, int N>
-__device__ __forceinline__ void screen_slices(const PairRec &pr, const PPStored &src, int pure,
-                                              double (&s)[ncart(LA) * ncart(LB)])
-{
-    constexpr int NA = ncart(LA), NB = ncart(LB), NR = LA + LB + 1;
-    if constexpr (CD0 < NA * NB) {
-        double acc[NA * NB * N];
-#pragma unroll
-        for (int k = 0; k < NA * NB * N; k++) acc[k] = 0.0;
-        eri_accumulate_cd<LA, LB, LA, LB, CD0, N, false>(src, pr, src, pr, acc, RysTab<double>::ptr(NR));
-        const int sa = nsph_of(LA, pure), sb = nsph_of(LB, pure);
-#pragma unroll
-        for (int m = 0; m < NA; m++) {
-#pragma unroll
-            for (int n = 0; n < NB; n++) {
-                if (m >= sa || n >= sb) continue;
-                double v = 0.0;
-#pragma unroll
-                for (int t = 0; t < N; t++) {
-                    const int k = (CD0 + t) % NA, l = (CD0 + t) / NA;
-                    const double tk = sph_coef(LA, pure, m, k), tl = sph_coef(LB, pure, n, l);
-                    if (tk == 0.0 || tl == 0.0) continue;
-#pragma unroll
-                    for (int i = 0; i < NA; i++) {
-                        const double ti = sph_coef(LA, pure, m, i);
-                        if (ti == 0.0) continue;
-#pragma unroll
-                        for (int j = 0; j < NB; j++) {
-                            const double tj = sph_coef(LB, pure, n, j);
-                            if (tj == 0.0) continue;
-                            v += ti * tj * tk * tl * acc[i + NA * (j + NB * t)];
-                        }
-                    }
-                }
-                s[m * NB + n] += v;
-            }
-        }
-        screen_slices<LA, LB, CD0 + N, N>(pr, src, pure, s);
-    }
-}
-
-// max |(mn|mn)| over the diagonal of (MN|MN) in the basis's own functions
-// (pfock/screening.c:59-90), for the pairs of one class
-template <int LA, int LB>
-__global__ void __launch_bounds__(64) k_screen(const PairRec *__restrict__ pairs, PrimPairs pp,
-                                               const int2 *__restrict__ mn, int n, int ns, int pure,
-                                               double *__restrict__ sq, unsigned long long *__restrict__ gmax)
-{
-    constexpr int NA = ncart(LA), NB = ncart(LB);
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const PairRec pr = pairs[t];
-    PPStored src{pp};
-    double s[NA * NB];
-#pragma unroll
-    for (int k = 0; k < NA * NB; k++) s[k] = 0.0;
-    screen_slices<LA, LB, 0, screen_slice_n(LA, LB)>(pr, src, pure, s);
-    const int sa = nsph_of(LA, pure), sb = nsph_of(LB, pure);
-    double mx = 0.0;
-#pragma unroll
-    for (int m = 0; m < NA; m++)
-#pragma unroll
-        for (int n2 = 0; n2 < NB; n2++)
-            if (m < sa && n2 < sb && fabs(s[m * NB + n2]) > mx) mx = fabs(s[m * NB + n2]);
-    const int M = mn[t].x, N = mn[t].y;
-    sq[(size_t)M * ns + N] = mx;
-    sq[(size_t)N * ns + M] = mx;
-    atomicMax(gmax, (unsigned long long)__double_as_longlong(mx));
-}
-
-static int launch_screen(int cls, const PairRec *pairs, PrimPairs pp, const int2 *mn, int n, int ns, int pure,
-                         double *sq, unsigned long long *gmax, cudaStream_t st)
-{
-    const unsigned g = (unsigned)((n + 63) / 64);
-    switch (cls) {
-        case 0: k_screen<0, 0><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-        case 1: k_screen<1, 0><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-        case 2: k_screen<1, 1><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-        case 3: k_screen<2, 0><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-        case 4: k_screen<2, 1><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-        case 5: k_screen<2, 2><<<g, 64, 0, st>>>(pairs, pp, mn, n, ns, pure, sq, gmax); break;
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
+// screen.cu: diagonal quartets of one class into sq and the maximum; sums is
+// scratch of ncart(la) * ncart(lb) doubles per pair
+int gtf_launch_screen(int la, int lb, const PairRec *pairs, PrimPairs pp, const int2 *mn, int n, int ns, int pure,
+                      double *sums, double *sq, unsigned long long *gmax, cudaStream_t st);
 
 // keep flag per (M, N): value > eta and the parity rule (pfock/screening.c:127-133)
 __global__ void k_csr_flags(const double *__restrict__ sq, int ns, double eta, int *__restrict__ flags)
@@ -842,11 +736,12 @@ __global__ void k_fill_pp32(const PairRec *__restrict__ pairs, int npairs, const
 // bound sqrt(v_i v_j) below the FP32 cutoff, form the tail of each prefix and
 // go to the FP32 launch; n64 counts the FP64 head.
 //
-// Per bra, the kets of all segments (in segment order, segment 0 left out)
-// form one list per launch part, so a warp's 32 lanes are filled across
-// segment boundaries: cum[i][b] is the exclusive prefix of the segment counts
-// and the bra has ceil(total / 32) units; the unit prefixes over the bras
-// close the lists.
+// Per bra, the kets of all segments (last segment first, segment 0 left out)
+// form one list of lanes per launch part, so a warp's 32 lanes are filled
+// across segment boundaries: a ket of segment b has the lanes gtf_lane_split
+// gives it, cum[i][q] is the exclusive prefix of the lanes of segment
+// GTF_NBKT - 1 - q, and the bra has ceil(total / 32) units; the unit prefixes
+// over the bras close the lists.
 //
 // The thresholds are an engine's static ones, or, for incremental builds,
 // read from the engine's device state, where they were scaled by the largest
@@ -856,6 +751,7 @@ __global__ void k_fill_pp32(const PairRec *__restrict__ pairs, int npairs, const
 // ---------------------------------------------------------------------------
 struct UnitTask {
     const double *pair_v;
+    const PairRec *pairs;
     int *nket, *n64, *cum64, *cum32;
     long long *up64, *up32;      // unit prefixes, [nbra + 1] each
     DynState *dyn;               // null: the static thresholds below
@@ -863,6 +759,7 @@ struct UnitTask {
     long long idx0;              // first (bra, segment) index of this task, over all tasks
     long long bra0;              // first bra index of this task, over all tasks
     int bra_start, nbra, ket_start, same;
+    int split_lt;                // lane split of long quartets (gtf_lane_split)
     int seg[GTF_NBKT + 1];
 };
 
@@ -935,14 +832,18 @@ __global__ void k_units_pack(const UnitTask *__restrict__ tasks, int nt, long lo
         const int k = task_of(tasks, nt, x, [](const UnitTask &t) { return t.bra0; });
         const UnitTask &t = tasks[k];
         const int i = (int)(x - t.bra0);
+        const int nbp = t.pairs[t.bra_start + i].n;
         int a = 0, c = 0;
-        for (int b = 0; b < GTF_NBKT; b++) {
-            t.cum64[i * GTF_CUM + b] = a;
-            t.cum32[i * GTF_CUM + b] = c;
+        for (int q = 0; q < GTF_NBKT; q++) {
+            const int b = GTF_NBKT - 1 - q;
+            t.cum64[i * GTF_CUM + q] = a;
+            t.cum32[i * GTF_CUM + q] = c;
             if (b == 0) continue;  // pairs whose primitive pairs were all screened out
             const int n = t.nket[i * GTF_NBKT + b], h = t.n64[i * GTF_NBKT + b];
-            a += h;
-            c += n - h;
+            int lk, lb;
+            gtf_lane_split(nbp, b, t.split_lt, lk, lb);
+            a += h << (lk + lb);
+            c += (n - h) << (lk + lb);
         }
         t.cum64[i * GTF_CUM + GTF_NBKT] = a;
         t.cum32[i * GTF_CUM + GTF_NBKT] = c;
@@ -1336,6 +1237,14 @@ extern "C" int gtf_basis_dev_create(const gtf_basis_view_t *b, gtf_fock_dev_t **
     return upload_basis(f, b);
 }
 
+// log2 of the primitive quartets a lane keeps when a quartet is dealt out to
+// several lanes.
+static int split_log2(const ClassPairTask &t, int nsm)
+{
+    const double w = (double)t.nbra * t.nketcls * (t.X == t.Y ? 0.5 : 1.0) / ((double)nsm * 512.0);
+    return w < 4 ? 4 : w < 16 ? 5 : 6;
+}
+
 // The engine's task set: one UnitTask per class pair with work, static and
 // dynamic copies on the device (called once, after the per-task arrays exist).
 static int make_unit_tasks(gtf_fock_dev *f)
@@ -1348,6 +1257,8 @@ static int make_unit_tasks(gtf_fock_dev *f)
         UnitTask u;
         memset(&u, 0, sizeof(u));
         u.pair_v = f->d_pair_v;
+        u.pairs = f->d_pairs;
+        u.split_lt = t.split_lt;
         u.nket = t.d_nket;
         u.n64 = t.d_n64;
         u.cum64 = t.d_cum64;
@@ -1385,18 +1296,18 @@ static int shard_bounds(gtf_fock_dev *f, int c, const std::vector<int> &nk, cons
 // Totals of one class pair's (bra, segment) ket counts: quartets, FP32
 // quartets and the bound on a launch's units (sum over bras of the units of
 // all non-empty segments).  64-bit integer sums: exact whatever the order.
-__global__ void k_unit_totals(const int *__restrict__ nk, const int *__restrict__ n64, int nbra,
+__global__ void k_unit_totals(const int *__restrict__ nk, const int *__restrict__ n64,
+                              const int *__restrict__ cum64, const int *__restrict__ cum32, int nbra,
                               unsigned long long *__restrict__ out)
 {
     unsigned long long q = 0, q32 = 0, bound = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nbra; i += gridDim.x * blockDim.x) {
-        long long all = 0;
+        const long long all = (long long)cum64[i * GTF_CUM + GTF_NBKT] + cum32[i * GTF_CUM + GTF_NBKT];
 #pragma unroll
         for (int b = 0; b < GTF_NBKT; b++) {
             const int k = i * GTF_NBKT + b;
             q += (unsigned long long)nk[k];
             q32 += (unsigned long long)(nk[k] - n64[k]);
-            if (b > 0) all += nk[k];
         }
         bound += (unsigned long long)((all + 31) / 32);
     }
@@ -1449,7 +1360,7 @@ static int build_units(gtf_fock_dev *f)
         const int nidx = t.nbra * GTF_NBKT;
         int g = (t.nbra + 255) / 256;
         if (g > 4 * f->nsm) g = 4 * f->nsm;
-        k_unit_totals<<<g, 256, 0, st>>>(t.d_nket, t.d_n64, t.nbra, f->d_unit_tot + 3 * c);
+        k_unit_totals<<<g, 256, 0, st>>>(t.d_nket, t.d_n64, t.d_cum64, t.d_cum32, t.nbra, f->d_unit_tot + 3 * c);
         CK(cudaGetLastError());
         nl++;
         CK(cudaMemcpyAsync(&t.nunits, t.d_unit_prefix + t.nbra, sizeof(long long), cudaMemcpyDeviceToHost, st));
@@ -1579,24 +1490,27 @@ extern "C" int gtf_fock_create(const gtf_basis_view_t *b, double tolscr, int max
             int2 *d_mn;
             int *d_off;
             PairRec *d_pr;
-            double *d_pp;
+            double *d_pp, *d_sums;
+            const int la = k_cls_la[c], lb = k_cls_lb[c];
             TALLOC(tmps, d_mn, n);
             TALLOC(tmps, d_off, n);
             TALLOC(tmps, d_pr, n);
             TALLOC(tmps, d_pp, 5 * npp_cls[c]);
+            TALLOC(tmps, d_sums, (size_t)n * ncart(la) * ncart(lb));
             CK(cudaMemcpyAsync(d_mn, mn[c].data(), sizeof(int2) * n, cudaMemcpyHostToDevice, st));
             CK(cudaMemcpyAsync(d_off, off[c].data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
             k_screen_prep<<<(n + 127) / 128, 128, 0, st>>>(bd, d_mn, d_off, n, d_pr, d_pp, npp_cls[c]);
             CK(cudaGetLastError());
             const size_t np_ = npp_cls[c];
             PrimPairs pps{d_pp, d_pp + np_, d_pp + 2 * np_, d_pp + 3 * np_, d_pp + 4 * np_};
-            if (launch_screen(c, d_pr, pps, d_mn, n, ns, b->pure, f->d_sq, d_gmax, st) != 0)
+            if (gtf_launch_screen(la, lb, d_pr, pps, d_mn, n, ns, b->pure, d_sums, f->d_sq, d_gmax, st) != 0)
                 CK(cudaGetLastError());
             CK(cudaStreamSynchronize(st));
             tmps.drop(d_mn);
             tmps.drop(d_off);
             tmps.drop(d_pr);
             tmps.drop(d_pp);
+            tmps.drop(d_sums);
         }
     }
     unsigned long long hmax = 0;
@@ -1727,6 +1641,7 @@ extern "C" int gtf_fock_create(const gtf_basis_view_t *b, double tolscr, int max
             for (int bk = 0; bk <= GTF_NBKT; bk++) t.seg[bk] = key_start[Y * 16 + bk] - t.ket_start;
             t.nunits = t.nunits32 = 0;
             t.nquart = t.nquart32 = 0.0;
+            t.split_lt = split_log2(t, f->nsm);
             if (t.nbra == 0 || t.nketcls == 0) continue;
             const int nidx = t.nbra * GTF_NBKT;
             DALLOC(t.d_nket, nidx);
@@ -2096,6 +2011,7 @@ static void fill_launch(const gtf_fock_dev *f, int c, int part, const double *D,
     a.unit_prefix = part ? t.d_unit_prefix32 : t.d_unit_prefix;
     a.nbra = t.nbra;
     a.nunits = part ? t.nunits32 : t.nunits;
+    a.split_lt = t.split_lt;
     a.bra_start = t.bra_start;
     a.ket_start = t.ket_start;
     for (int b = 0; b <= GTF_NBKT; b++) a.seg[b] = t.seg[b];

@@ -32,6 +32,35 @@ __host__ __device__ inline int gtf_prim_bucket(int n)
     return 14;
 }
 
+// floor(log2) of the fewest primitive pairs of a pair in bucket b (0 for
+// bucket 0, which gets no units): 0 0 1 1 2 2 3 3 4 4 4 5 5 5 6, three bits each
+#define GTF_BUCKET_LOG2 0x1adb246d2240ULL
+__host__ __device__ inline int gtf_bucket_log2(int b) { return (int)(GTF_BUCKET_LOG2 >> (3 * b)) & 7; }
+__host__ __device__ inline int gtf_log2_floor(int x)
+{
+#ifdef __CUDA_ARCH__
+    return 31 - __clz(x);
+#else
+    int l = 0;
+    while (x >>= 1) l++;
+    return l;
+#endif
+}
+
+// Lanes sharing one quartet, 2^(lk + lb) <= 32: the ket primitives are dealt
+// out to 2^lk lanes and the bra primitives to 2^lb, so that a lane keeps about
+// 2^lt primitive quartets or more.  The count does not decrease with the
+// bucket: a bra's kets, laid out from the highest bucket down, start every
+// group at a multiple of its size.
+__host__ __device__ inline void gtf_lane_split(int nbraprim, int b, int lt, int &lk, int &lb)
+{
+    const int mk = gtf_bucket_log2(b), mb = gtf_log2_floor(nbraprim | 1);
+    int l = mk + mb - lt;
+    l = l < 0 ? 0 : l > 5 ? 5 : l;
+    lk = mk < l ? mk : l;
+    lb = l - lk;   // <= mb, since l <= mk + mb
+}
+
 // One molecule's part of a class-pair launch (its task lists, pair data, D
 // and accumulators).
 struct FockLaunch {
@@ -39,8 +68,8 @@ struct FockLaunch {
     const double2 *pprec;          // primitive-pair records (PPRec)
     const float4 *pprec32;         // FP32 primitive-pair records (PPRec32)
     const int *nlo;                // [nbra][GTF_NBKT] first ket of this launch in each segment prefix (null: 0)
-    const int *cum;                // [nbra][GTF_CUM] exclusive prefix over segments of this launch's kets
-    const long long *unit_prefix;  // [nbra + 1] exclusive prefix of units (32 kets) over bras
+    const int *cum;                // [nbra][GTF_CUM] exclusive prefix of lanes over segments, last segment first
+    const long long *unit_prefix;  // [nbra + 1] exclusive prefix of units (32 lanes) over bras
     int nbra;
     long long nunits;
     int bra_start, ket_start;
@@ -48,6 +77,7 @@ struct FockLaunch {
     const double *D;
     double *Fj, *Fk;
     int ld;
+    int split_lt;                  // lane split of long quartets (gtf_lane_split)
     int konly;                     // exchange terms only (antisymmetric part of a non-symmetric D)
 };
 
@@ -120,7 +150,7 @@ __global__ void __launch_bounds__(FOCK_THREADS,
     constexpr int NCD = ncart(LC) * ncart(LD);
     constexpr int S = fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
     constexpr int N = (NCD - CD0 < S) ? NCD - CD0 : S;
-    __shared__ __align__(16) R tab[RysTab<R>::slen(NR)];
+    __shared__ __align__(16) R tab[RysTab<R>::len(NR)];
     // the launch's unit count, kept in shared memory rather than a register
     // across the integral loops (visible after the staging's barrier)
     __shared__ unsigned long long s_nunits;
@@ -156,7 +186,7 @@ __global__ void __launch_bounds__(FOCK_THREADS,
                 uend = u + claim;
             }
             if (u >= *(volatile unsigned long long *)&s_nunits) break;
-            uu = u;
+            uu = *(volatile unsigned long long *)&s_nunits - 1 - u;   // last bras, the longest, first
             __syncwarp();
             if (lane == 0) {
                 sc[0] = u + 1;
@@ -168,7 +198,7 @@ __global__ void __launch_bounds__(FOCK_THREADS,
             if (lane == 0) c0 = atomicAdd(counter, 1ULL);
             uu = __shfl_sync(GTF_FULL_MASK, c0, 0);
             if (uu >= *(volatile unsigned long long *)&s_nunits) break;
-            uu += (unsigned long long)g.unit_lo;
+            uu = *(volatile unsigned long long *)&s_nunits - 1 - uu + (unsigned long long)g.unit_lo;
         }
         // molecule of the unit (batched launches); the fields are read from
         // the kernel parameter (one molecule, no registers held for them) or
@@ -185,10 +215,10 @@ __global__ void __launch_bounds__(FOCK_THREADS,
         }
 #define GTF_FLD(x) (bt ? mp->x : g.one.x)
         const long long *unit_prefix = GTF_FLD(unit_prefix);
-        // unit u -> (bra i, chunk of 32 kets) by a warp search of the unit
+        // unit u -> (bra i, chunk of 32 lanes) by a warp search of the unit
         // prefix over bras; lane v of the chunk -> segment b and position in
         // it from the bra's segment prefix (the kets of consecutive segments
-        // share a warp)
+        // share a warp); a quartet of many primitives has 2^(lk + lb) lanes
         const int nbra = GTF_FLD(nbra);
         const int i = warp_find_le(unit_prefix, nbra, (long long)uu, lane);
         const int v = (int)((long long)uu - __ldg(unit_prefix + i)) * 32 + lane;
@@ -197,19 +227,24 @@ __global__ void __launch_bounds__(FOCK_THREADS,
         const int cum[GTF_CUM] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w,
                                   c2.x, c2.y, c2.z, c2.w, c3.x, c3.y, c3.z, c3.w};
         const bool active = v < cum[GTF_NBKT];
-        int b = 0, cb = 0;
+        int b = GTF_NBKT - 1, cb = 0;
 #pragma unroll
         for (int k = 1; k < GTF_NBKT; k++)
             if (cum[k] <= v) {
-                b = k;
+                b = GTF_NBKT - 1 - k;
                 cb = cum[k];
             }
         const int *nlo = GTF_FLD(nlo);
         const int k0 = nlo ? __ldg(nlo + (size_t)i * GTF_NBKT + b) : 0;
-        const int j = GTF_FLD(seg[b]) + k0 + (v - cb);
         const PairRec *pairs = GTF_FLD(pairs);
         const int bra_start = GTF_FLD(bra_start), ket_start = GTF_FLD(ket_start);
         const PairRec pb = pairs[bra_start + i];
+        int lk, lb;
+        gtf_lane_split(pb.n, b, GTF_FLD(split_lt), lk, lb);
+        if (!active) lk = lb = 0;
+        const int sub = (v - cb) & ((1 << (lk + lb)) - 1);
+        const int split = prim_split(1 << lk, sub & ((1 << lk) - 1), 1 << lb, sub >> lk);
+        const int j = GTF_FLD(seg[b]) + k0 + ((v - cb) >> (lk + lb));
         const PairRec pk = active ? pairs[ket_start + j] : pb;
         const bool same = (bra_start + i) == (ket_start + j);
         R acc[ncart(LA) * ncart(LB) * N];
@@ -217,13 +252,24 @@ __global__ void __launch_bounds__(FOCK_THREADS,
         for (int k = 0; k < ncart(LA) * ncart(LB) * N; k++) acc[k] = (R)0;
         if constexpr (sizeof(R) == 4) {
             const PPRec32 src{GTF_FLD(pprec32)};
-            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true, true>(src, pb, pk, acc, tab);
+            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true>(src, pb, pk, acc, tab, split);
         } else {
             const PPRec src{GTF_FLD(pprec)};
-            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true, true>(src, pb, src, pk, acc, tab);
+            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true>(src, pb, src, pk, acc, tab, split);
         }
+        // sum the lanes of each quartet; the first of them digests it
+        const int nl = (split & 0xff) * ((split >> 8) & 0xff);
+        const int nlmax = __reduce_max_sync(GTF_FULL_MASK, nl);
+        for (int o = 1; o < nlmax; o <<= 1) {
+#pragma unroll
+            for (int k = 0; k < ncart(LA) * ncart(LB) * N; k++) {
+                const R t = __shfl_xor_sync(GTF_FULL_MASK, acc[k], o);
+                if (o < nl) acc[k] += t;
+            }
+        }
+        const bool digest = active && (split >> 16) == 0;
         if constexpr (BATCH) mp = g.mols + ((volatile int *)s_mol)[wib];   // reloaded after the loops
-        digest_cd<LA, LB, LC, LD, CD0, N>(acc, active, pb, pk, same, GTF_FLD(D), GTF_FLD(Fj), GTF_FLD(Fk),
+        digest_cd<LA, LB, LC, LD, CD0, N>(acc, digest, pb, pk, same, GTF_FLD(D), GTF_FLD(Fj), GTF_FLD(Fk),
                                           GTF_FLD(ld), lane, GTF_FLD(konly) != 0);
 #undef GTF_FLD
     }

@@ -3,7 +3,7 @@
 // Replaces the integral engine behind CInt_computeShellQuartet
 // (libcint/include/CInt.h:159-167, called at pfock/fock_task.c:197-198) and
 // the J/K digestion update_F (pfock/fock_task.c:29-117):
-//   * rys_roots<N>: N-point Rys quadrature for the Boys weight from the
+//   * RysArg<N>: N-point Rys quadrature for the Boys weight from the
 //     generated Chebyshev-fitted table (rys_table.h), large-T Hermite form;
 //   * eri_accumulate<LA,LB,LC,LD>: contracted Cartesian (ab|cd) by Rys
 //     quadrature -- per primitive quartet and root the 2-D integrals
@@ -139,139 +139,137 @@ __host__ __device__ constexpr int rys_deg(int n)
 }
 
 // The N-root block of each table is [off(N), off(N+1)); its extent is known
-// at compile time so kernels can stage it in shared memory.  rows(N) values
-// per interval; a lane reads one interval's row as 2-value vectors (16 bytes
-// FP64, 8 bytes FP32).  The lanes of a warp read different intervals, so the
-// shared-memory copy pads each interval to srows(N), an odd number of vectors:
-// consecutive intervals then start in different banks (unpadded, the FP64
-// 4-root rows are 48 vectors long and every interval starts in the same bank).
+// at compile time so kernels can stage it in shared memory.  An interval is
+// stride(N) values of pairs (u_r, w_r), an odd number of pairs (16 bytes FP64,
+// 8 bytes FP32): the lanes of a warp read different intervals, and
+// consecutive ones then start in different banks.
 template <typename R>
 struct RysTab;
 template <>
 struct RysTab<double> {
+    typedef double2 V2;
     static __host__ __device__ constexpr int off(int n)
     {
         constexpr int o[] = {RYS_OFF_LIST, RYS_TABLE_LEN};
         return o[n];
     }
     static __host__ __device__ constexpr int len(int n) { return off(n + 1) - off(n); }
-    static __host__ __device__ constexpr int rows(int n) { return (rys_deg(n) + 1) * 2 * n; }
-    static __host__ __device__ constexpr int srows(int n) { return (rows(n) / 2) % 2 == 0 ? rows(n) + 2 : rows(n); }
-    static __host__ __device__ constexpr int slen(int n) { return len(n) / rows(n) * srows(n); }
+    static __host__ __device__ constexpr int deg(int n) { return rys_deg(n); }
+    static __host__ __device__ constexpr double h(int n) { return rys_h(n); }
+    static __host__ __device__ constexpr int stride(int n) { return 2 * ((deg(n) + 1) * n | 1); }
     static __device__ __forceinline__ const double *ptr(int n) { return RYS_TABLE + off(n); }
 };
 template <>
 struct RysTab<float> {
+    typedef float2 V2;
     static __host__ __device__ constexpr int off(int n)
     {
         constexpr int o[] = {RYS32_OFF_LIST, RYS32_TABLE_LEN};
         return o[n];
     }
     static __host__ __device__ constexpr int len(int n) { return off(n + 1) - off(n); }
-    static __host__ __device__ constexpr int rows(int n) { return (RYS32_DEG + 1) * 2 * n; }
-    static __host__ __device__ constexpr int srows(int n) { return (rows(n) / 2) % 2 == 0 ? rows(n) + 2 : rows(n); }
-    static __host__ __device__ constexpr int slen(int n) { return len(n) / rows(n) * srows(n); }
+    static __host__ __device__ constexpr int deg(int) { return RYS32_DEG; }
+    static __host__ __device__ constexpr float h(int) { return (float)RYS32_H; }
+    static __host__ __device__ constexpr int stride(int n) { return 2 * ((deg(n) + 1) * n | 1); }
     static __device__ __forceinline__ const float *ptr(int n) { return RYS32_TABLE + off(n); }
 };
 
-// Stages the N-root block into shared memory with the padded row stride.
+// Stages the N-root block into shared memory: 16-byte asynchronous copies,
+// all in flight at once.  (A loop of 8-byte loads was one dependent round
+// trip to L2 per thread and pass, up to 46 of them: most of the time of a
+// launch with little work.)
 template <typename R, int N>
 __device__ __forceinline__ void rys_stage(R *stab)
 {
-    constexpr int RW = RysTab<R>::rows(N), SR = RysTab<R>::srows(N), TL = RysTab<R>::len(N);
-    static_assert(TL % RW == 0, "whole intervals");
-    const R *gt = RysTab<R>::ptr(N);
-    for (int k = threadIdx.x; k < TL; k += blockDim.x) stab[(k / RW) * SR + k % RW] = __ldg(gt + k);
+    constexpr int NV = RysTab<R>::len(N) * (int)sizeof(R) / 16;
+    static_assert(RysTab<R>::len(N) * sizeof(R) % 16 == 0 && RysTab<R>::off(N) * sizeof(R) % 16 == 0, "whole vectors");
+    const char *src = reinterpret_cast<const char *>(RysTab<R>::ptr(N));
+    const unsigned dst = (unsigned)__cvta_generic_to_shared(stab);
+    for (int k = threadIdx.x; k < NV; k += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * k), "l"(src + 16 * k) : "memory");
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     __syncthreads();
 }
 
-// tab: the N-root block of RYS_TABLE (global, STRIDE = rows) or its padded
-// shared-memory copy (STRIDE = srows)
-template <int N, int STRIDE = RysTab<double>::rows(N)>
-__device__ __forceinline__ void rys_roots(double T, double (&u)[N], double (&w)[N], const double *tab)
-{
-    constexpr double H = rys_h(N), INV_H = 1.0 / rys_h(N);
-    constexpr int DEG = rys_deg(N);
-    if (T >= RYS_TMAX[N]) {
-        const double it = 1.0 / T;
-        const double rs = rsqrt(T);
+// Roots and weights of one argument T: below RYS_TMAX the interval's
+// polynomials in s (a degree-7 fit in FP32, the FP64 table's degrees
+// otherwise), above it the large-T form.  tab: the N-root block of the global
+// table or its copy in shared memory.  all() evaluates every root at once,
+// root() one of them.
+template <int N, typename R>
+struct RysArg {
+    R a, b;         // s and -, or 1/T and 1/sqrt(T)
+    const R *row;   // the interval's coefficients; null: large T
+    __device__ __forceinline__ RysArg(R T, const R *tab)
+    {
+        constexpr R H = RysTab<R>::h(N), INV_H = (R)1 / RysTab<R>::h(N);
+        if (T >= (R)RYS_TMAX[N]) {
+            a = (R)1 / T;
+            b = grsqrt(T);
+            row = nullptr;
+        } else {
+            const int k = (int)(T * INV_H);
+            a = T - ((R)k * H + (R)0.5 * H);
+            b = (R)0;
+            row = tab + k * RysTab<R>::stride(N);
+        }
+    }
+    __device__ __forceinline__ void all(R (&u)[N], R (&w)[N]) const
+    {
+        constexpr int DEG = RysTab<R>::deg(N);
+        if (row == nullptr) {
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                u[i] = (R)RYS_LARGE_X2[N][i] * a;
+                w[i] = (R)RYS_LARGE_W[N][i] * b;
+            }
+            return;
+        }
+        typedef typename RysTab<R>::V2 V2;
+        const V2 *c2 = reinterpret_cast<const V2 *>(row);
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            u[i] = RYS_LARGE_X2[N][i] * it;
-            w[i] = RYS_LARGE_W[N][i] * rs;
+            const V2 t = c2[DEG * N + i];
+            u[i] = t.x;
+            w[i] = t.y;
         }
-        return;
-    }
-    const int k = (int)(T * INV_H);
-    const double s = T - ((double)k * H + 0.5 * H);
-    static_assert(STRIDE % 2 == 0 && STRIDE >= (DEG + 1) * 2 * N, "interval stride");
-    const double *c = tab + k * STRIDE;
-    // rows of 2N coefficients start on 16-byte boundaries (even offsets)
-    const double2 *c2 = reinterpret_cast<const double2 *>(c);
-    double a[2 * N];
 #pragma unroll
-    for (int f = 0; f < N; f++) {
-        const double2 t = c2[DEG * N + f];
-        a[2 * f] = t.x;
-        a[2 * f + 1] = t.y;
-    }
+        for (int j = DEG - 1; j >= 0; j--) {
 #pragma unroll
-    for (int j = DEG - 1; j >= 0; j--) {
-#pragma unroll
-        for (int f = 0; f < N; f++) {
-            const double2 t = c2[j * N + f];
-            a[2 * f] = fma(a[2 * f], s, t.x);
-            a[2 * f + 1] = fma(a[2 * f + 1], s, t.y);
+            for (int i = 0; i < N; i++) {
+                const V2 t = c2[j * N + i];
+                u[i] = gfma(u[i], a, t.x);
+                w[i] = gfma(w[i], a, t.y);
+            }
         }
     }
+    __device__ __forceinline__ void root(int r, R &u, R &w) const
+    {
+        constexpr int DEG = RysTab<R>::deg(N);
+        if (row == nullptr) {
+            u = (R)RYS_LARGE_X2[N][r] * a;
+            w = (R)RYS_LARGE_W[N][r] * b;
+            return;
+        }
+        typedef typename RysTab<R>::V2 V2;
+        const V2 *c2 = reinterpret_cast<const V2 *>(row) + r;
+        const V2 t0 = c2[DEG * N];
+        u = t0.x;
+        w = t0.y;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
-        u[i] = a[i];
-        w[i] = a[N + i];
+        for (int j = DEG - 1; j >= 0; j--) {
+            const V2 t = c2[j * N];
+            u = gfma(u, a, t.x);
+            w = gfma(w, a, t.y);
+        }
     }
-}
+};
 
-// FP32 form for quartets evaluated in single precision: degree-7 fit of the
-// same functions on the same intervals (RYS32_TABLE), same large-T form
-template <int N, int STRIDE = RysTab<float>::rows(N)>
-__device__ __forceinline__ void rys_roots(float T, float (&u)[N], float (&w)[N], const float *tab)
-{
-    if (T >= (float)RYS_TMAX[N]) {
-        const float it = 1.0f / T;
-        const float rs = rsqrtf(T);
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            u[i] = (float)RYS_LARGE_X2[N][i] * it;
-            w[i] = (float)RYS_LARGE_W[N][i] * rs;
-        }
-        return;
-    }
-    const int k = (int)(T * RYS32_INV_H);
-    const float s = T - ((float)k * (float)RYS32_H + 0.5f * (float)RYS32_H);
-    static_assert(STRIDE % 2 == 0 && STRIDE >= (RYS32_DEG + 1) * 2 * N, "interval stride");
-    const float2 *c2 = reinterpret_cast<const float2 *>(tab + k * STRIDE);
-    float a[2 * N];
-#pragma unroll
-    for (int f = 0; f < N; f++) {
-        const float2 t = c2[RYS32_DEG * N + f];
-        a[2 * f] = t.x;
-        a[2 * f + 1] = t.y;
-    }
-#pragma unroll
-    for (int j = RYS32_DEG - 1; j >= 0; j--) {
-#pragma unroll
-        for (int f = 0; f < N; f++) {
-            const float2 t = c2[j * N + f];
-            a[2 * f] = fmaf(a[2 * f], s, t.x);
-            a[2 * f + 1] = fmaf(a[2 * f + 1], s, t.y);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++) {
-        u[i] = a[i];
-        w[i] = a[N + i];
-    }
-}
+// (dd| quartets keep the roots a loop: the unrolled body of 36 to 72
+// integrals times 3 to 5 roots outgrows the instruction caches.  On C54H18 /
+// cc-pVDZ the loop took (dd|dp) from 8.5 to 7.2 ms and (dd|pp) from 6.9 to
+// 5.9 ms; the other classes were 2-6% slower with it.
+__host__ __device__ constexpr bool rys_loop(int lab) { return lab >= 4; }
 
 // ---------------------------------------------------------------------------
 // one-dimensional horizontal transfer:
@@ -356,6 +354,13 @@ __device__ __forceinline__ void hrr_abcd(const R (&G)[LA + LB + 1][LC + LD + 1],
 // ---------------------------------------------------------------------------
 // contracted Cartesian (ab|cd), accumulated into acc[ia + NA*(ib + NB*(ic + NC*id))]
 // ---------------------------------------------------------------------------
+// A lane's share of a quartet's primitive loops: ket primitives k0, k0 + ks,
+// ... and bra primitives b0, b0 + bs, ... (ks * bs lanes share the quartet),
+// packed into one register across the loops.
+__host__ __device__ constexpr int prim_split(int ks, int k0, int bs, int b0)
+{
+    return ks | (bs << 8) | (k0 << 16) | (b0 << 24);
+}
 // SKIP: primitive pairs are sorted by descending |K| (Fock-build pair list),
 // so the primitive-quartet cutoff may end the ket loop early
 // Restricted to the ket components cd = CD0 .. CD0+N-1 (cd = ic + NC*id):
@@ -367,32 +372,33 @@ __device__ __forceinline__ void hrr_abcd(const R (&G)[LA + LB + 1][LC + LD + 1],
 // Loop order: ket primitive pairs outside (one per lane), bra primitive pairs
 // inside -- the bra is shared by the warp, so its records are warp-uniform
 // loads that stay in L1, and each lane reads its ket's records once.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool SPAD = false, class PPB, class PPK,
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, class PPB, class PPK,
           typename R>
 __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec &pb, const PPK &ket,
                                                   const PairRec &pk, R (&acc)[ncart(LA) * ncart(LB) * N],
-                                                  const R *rtab)
+                                                  const R *rtab, int split = prim_split(1, 0, 1, 0))
 {
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    if (pb.n <= 0) return;
     const R ABx = (R)pb.ABx, ABy = (R)pb.ABy, ABz = (R)pb.ABz;
     const R CDx = (R)pk.ABx, CDy = (R)pk.ABy, CDz = (R)pk.ABz;
-    const PrimVals b0 = bra.get(pb, 0);
+    const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
+    if (ib0 >= pb.n) return;
+    const PrimVals b0 = bra.get(pb, ib0);
     PrimVals nk;
-    if (pk.n > 0) nk = ket.get(pk, 0);
-    for (int ik = 0; ik < pk.n; ik++) {
+    if (ik0 < pk.n) nk = ket.get(pk, ik0);
+    for (int ik = ik0; ik < pk.n; ik += kstep) {
         const PrimVals kq = nk;
-        if (ik + 1 < pk.n) nk = ket.get(pk, ik + 1);
+        if (ik + kstep < pk.n) nk = ket.get(pk, ik + kstep);
         if (SKIP && fabs(b0.K * kq.K) < GTF_PRIMQ_EPS) break;  // both lists are in descending |K|
         const R q_ = (R)kq.p, h2q = (R)kq.h;
         const R QCx = (R)(kq.Px - pk.Ax), QCy = (R)(kq.Py - pk.Ay), QCz = (R)(kq.Pz - pk.Az);
         // the next bra primitive pair is loaded while the current one is used
         PrimVals nb = b0;
-        for (int ib = 0; ib < pb.n; ib++) {
+        for (int ib = ib0; ib < pb.n; ib += bstep) {
             const PrimVals bq = nb;
-            if (ib + 1 < pb.n) nb = bra.get(pb, ib + 1);
+            if (ib + bstep < pb.n) nb = bra.get(pb, ib + bstep);
             if (SKIP && fabs(bq.K * kq.K) < GTF_PRIMQ_EPS) break;
             const R p_ = (R)bq.p, h2p = (R)bq.h;
             const R PAx = (R)(bq.Px - pb.Ax), PAy = (R)(bq.Py - pb.Ay), PAz = (R)(bq.Pz - pb.Az);
@@ -402,12 +408,20 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
             const R rho = p_ * q_ * ipq;
             const R T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
             const R pref = (R)(bq.K * kq.K) * rpq;
+            const RysArg<NR, R> rys(T, rtab);
+            constexpr bool LOOP = rys_loop(LA + LB);
             R u[NR], w[NR];
-            rys_roots<NR, SPAD ? RysTab<R>::srows(NR) : RysTab<R>::rows(NR)>(T, u, w, rtab);
+            if constexpr (!LOOP) rys.all(u, w);
             const R qf = q_ * ipq, pf = p_ * ipq;
-#pragma unroll
+#pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
-                const R ur = u[r];
+                R ur, wr;
+                if constexpr (LOOP) {
+                    rys.root(r, ur, wr);
+                } else {
+                    ur = u[r];
+                    wr = w[r];
+                }
                 const R B00 = (R)0.5 * ur * ipq;
                 const R B10 = h2p * ((R)1 - qf * ur);
                 const R B01 = h2q * ((R)1 - pf * ur);
@@ -415,7 +429,7 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
                 R Gx[NI][NK], Gy[NI][NK], Gz[NI][NK];
                 rys_2d<NI, NK>(Gx, (R)1, PAx - cq * PQx, QCx + cp * PQx, B10, B01, B00);
                 rys_2d<NI, NK>(Gy, (R)1, PAy - cq * PQy, QCy + cp * PQy, B10, B01, B00);
-                rys_2d<NI, NK>(Gz, w[r] * pref, PAz - cq * PQz, QCz + cp * PQz, B10, B01, B00);
+                rys_2d<NI, NK>(Gz, wr * pref, PAz - cq * PQz, QCz + cp * PQz, B10, B01, B00);
                 R Ix[LA + 1][LB + 1][LC + 1][LD + 1];
                 R Iy[LA + 1][LB + 1][LC + 1][LD + 1];
                 R Iz[LA + 1][LB + 1][LC + 1][LD + 1];
@@ -445,31 +459,33 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
 // FP32 quartets: everything in single precision, from the FP32 records (centres
 // relative to each pair's first shell; P - Q = PA - QC + (A - C) with A - C
 // formed in double once per quartet).  Same structure as eri_accumulate_cd.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool SPAD = false>
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP>
 __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const PairRec &pb, const PairRec &pk,
-                                                    float (&acc)[ncart(LA) * ncart(LB) * N], const float *rtab)
+                                                    float (&acc)[ncart(LA) * ncart(LB) * N], const float *rtab,
+                                                    int split = prim_split(1, 0, 1, 0))
 {
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC);
-    if (pb.n <= 0) return;
     const float ABx = (float)pb.ABx, ABy = (float)pb.ABy, ABz = (float)pb.ABz;
     const float CDx = (float)pk.ABx, CDy = (float)pk.ABy, CDz = (float)pk.ABz;
     const float ACx = (float)(pb.Ax - pk.Ax), ACy = (float)(pb.Ay - pk.Ay), ACz = (float)(pb.Az - pk.Az);
-    const PrimVals32 b0 = src.get(pb, 0);
+    const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
+    if (ib0 >= pb.n) return;
+    const PrimVals32 b0 = src.get(pb, ib0);
     PrimVals32 nk;
-    if (pk.n > 0) nk = src.get(pk, 0);
-    for (int ik = 0; ik < pk.n; ik++) {
+    if (ik0 < pk.n) nk = src.get(pk, ik0);
+    for (int ik = ik0; ik < pk.n; ik += kstep) {
         const PrimVals32 kq = nk;
-        if (ik + 1 < pk.n) nk = src.get(pk, ik + 1);
+        if (ik + kstep < pk.n) nk = src.get(pk, ik + kstep);
         if (SKIP && fabsf(b0.K * kq.K) < (float)GTF_PRIMQ_EPS) break;
         const float q = kq.p, h2q = kq.h;
         const float QCx = kq.PAx, QCy = kq.PAy, QCz = kq.PAz;
         const float dx = ACx - QCx, dy = ACy - QCy, dz = ACz - QCz;
         PrimVals32 nb = b0;
-        for (int ib = 0; ib < pb.n; ib++) {
+        for (int ib = ib0; ib < pb.n; ib += bstep) {
             const PrimVals32 bq = nb;
-            if (ib + 1 < pb.n) nb = src.get(pb, ib + 1);
+            if (ib + bstep < pb.n) nb = src.get(pb, ib + bstep);
             if (SKIP && fabsf(bq.K * kq.K) < (float)GTF_PRIMQ_EPS) break;
             const float p = bq.p, h2p = bq.h;
             const float PAx = bq.PAx, PAy = bq.PAy, PAz = bq.PAz;
@@ -479,12 +495,20 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
             const float rho = p * q * ipq;
             const float T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
             const float pref = bq.K * kq.K * rpq;
+            const RysArg<NR, float> rys(T, rtab);
+            constexpr bool LOOP = rys_loop(LA + LB);
             float u[NR], w[NR];
-            rys_roots<NR, SPAD ? RysTab<float>::srows(NR) : RysTab<float>::rows(NR)>(T, u, w, rtab);
+            if constexpr (!LOOP) rys.all(u, w);
             const float qf = q * ipq, pf = p * ipq;
-#pragma unroll
+#pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
-                const float ur = u[r];
+                float ur, wr;
+                if constexpr (LOOP) {
+                    rys.root(r, ur, wr);
+                } else {
+                    ur = u[r];
+                    wr = w[r];
+                }
                 const float B00 = 0.5f * ur * ipq;
                 const float B10 = h2p * (1.0f - qf * ur);
                 const float B01 = h2q * (1.0f - pf * ur);
@@ -492,7 +516,7 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
                 float Gx[NI][NK], Gy[NI][NK], Gz[NI][NK];
                 rys_2d<NI, NK>(Gx, 1.0f, PAx - cq * PQx, QCx + cp * PQx, B10, B01, B00);
                 rys_2d<NI, NK>(Gy, 1.0f, PAy - cq * PQy, QCy + cp * PQy, B10, B01, B00);
-                rys_2d<NI, NK>(Gz, w[r] * pref, PAz - cq * PQz, QCz + cp * PQz, B10, B01, B00);
+                rys_2d<NI, NK>(Gz, wr * pref, PAz - cq * PQz, QCz + cp * PQz, B10, B01, B00);
                 float Ix[LA + 1][LB + 1][LC + 1][LD + 1];
                 float Iy[LA + 1][LB + 1][LC + 1][LD + 1];
                 float Iz[LA + 1][LB + 1][LC + 1][LD + 1];
