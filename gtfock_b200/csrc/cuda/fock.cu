@@ -109,6 +109,94 @@ struct ClassPairTask {
     long long *d_unit_prefix32;  // [nbra + 1], FP32 launch
 };
 
+// Side streams for the launches of one build, which are independent of one
+// another: fork() lets the first n - 1 of them start where fs.s[0] stands,
+// join() lets fs.s[0] go on once they are through.  The sets come from a
+// process-wide pool (creating one takes 0.3 ms) and return to it with the
+// engine or batch that took them, at most GTF_SIDE_SETS waiting there; a set
+// that returns has been joined, so whoever takes it next only queues behind
+// work that its former owner has waited for.
+#define GTF_SIDE_SETS 16
+struct SideStreams {
+    int dev;
+    cudaStream_t s[GTF_FOCK_STREAMS - 1];
+    cudaEvent_t ev_fork, ev_join[GTF_FOCK_STREAMS - 1];
+};
+static std::mutex g_side_mu;
+static std::vector<SideStreams *> g_side;
+
+static void side_destroy(SideStreams *p)
+{
+    for (int k = 0; k < GTF_FOCK_STREAMS - 1; k++) {
+        if (p->ev_join[k]) cudaEventDestroy(p->ev_join[k]);
+        if (p->s[k]) cudaStreamDestroy(p->s[k]);
+    }
+    if (p->ev_fork) cudaEventDestroy(p->ev_fork);
+    delete p;
+}
+
+struct ForkJoin {
+    SideStreams *p;
+    cudaError_t fork(FockStreams &fs, int n)
+    {
+        cudaError_t e = p ? cudaSuccess : take();
+        if (e == cudaSuccess) e = cudaEventRecord(p->ev_fork, fs.s[0]);
+        fs.n = n < 1 ? 1 : n > GTF_FOCK_STREAMS ? GTF_FOCK_STREAMS : n;
+        for (int k = 1; k < fs.n && e == cudaSuccess; k++) {
+            fs.s[k] = p->s[k - 1];
+            e = cudaStreamWaitEvent(fs.s[k], p->ev_fork, 0);
+        }
+        return e;
+    }
+    cudaError_t join(FockStreams &fs)
+    {
+        cudaError_t e = cudaSuccess;
+        for (int k = 1; k < fs.n && e == cudaSuccess; k++) {
+            e = cudaEventRecord(p->ev_join[k - 1], fs.s[k]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(fs.s[0], p->ev_join[k - 1], 0);
+        }
+        return e;
+    }
+    cudaError_t take()
+    {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        {
+            std::lock_guard<std::mutex> lk(g_side_mu);
+            for (size_t k = 0; k < g_side.size(); k++)
+                if (g_side[k]->dev == dev) {
+                    p = g_side[k];
+                    g_side.erase(g_side.begin() + k);
+                    return cudaSuccess;
+                }
+        }
+        SideStreams *q = new SideStreams();
+        q->dev = dev;
+        e = cudaEventCreateWithFlags(&q->ev_fork, cudaEventDisableTiming);
+        for (int k = 0; k < GTF_FOCK_STREAMS - 1 && e == cudaSuccess; k++) {
+            e = cudaStreamCreateWithFlags(&q->s[k], cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&q->ev_join[k], cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess) p = q;
+        else side_destroy(q);
+        return e;
+    }
+    void give_back()
+    {
+        if (!p) return;
+        {
+            std::lock_guard<std::mutex> lk(g_side_mu);
+            if (g_side.size() < GTF_SIDE_SETS) {
+                g_side.push_back(p);
+                p = nullptr;
+            }
+        }
+        if (p) side_destroy(p);
+        p = nullptr;
+    }
+};
+
 struct gtf_fock_dev {
     int dev;
     int nsm;
@@ -145,7 +233,8 @@ struct gtf_fock_dev {
     size_t host_stage_bytes;
     // timing
     cudaEvent_t ev0, ev1, ev2, ev3;
-    cudaEvent_t ev_cls[NCLSPAIR + 1];
+    cudaEvent_t ev_cls[2 * NCLSPAIR];   // start and end of each class pair's launches
+    ForkJoin side;
     double ms_total, ms_eri, ms_other;
     double ms_cls[NCLSPAIR];
     int prec;
@@ -943,11 +1032,11 @@ static int run_units(const UnitTask *d_tasks, int nt, long long nidx, long long 
     return GTF_OK;
 }
 
-typedef int (*fock_group_launch_t)(int la, int lb, int lc, int ld, const FockGrid &g, cudaStream_t st);
+typedef int (*fock_group_launch_t)(int la, int lb, int lc, int ld, const FockGrid &g, FockStreams &st);
 extern fock_group_launch_t gtf_fock_groups[];
 extern const int gtf_fock_ngroups;
 
-static int launch_fock(int X, int Y, const FockGrid &fg, cudaStream_t st)
+static int launch_fock(int X, int Y, const FockGrid &fg, FockStreams &st)
 {
     for (int g = 0; g < gtf_fock_ngroups; g++) {
         int r = gtf_fock_groups[g](k_cls_la[X], k_cls_lb[X], k_cls_la[Y], k_cls_lb[Y], fg, st);
@@ -1108,8 +1197,9 @@ static void tune_apply(int kind, int X, int Y, int part, FockGrid &g)
 static double tune_launch(int kind, int X, int Y, int part, FockGrid g, cudaStream_t st, int reps,
                           cudaEvent_t e0, cudaEvent_t e1)
 {
+    FockStreams one(st);
     g.query = 1;
-    const int occ = launch_fock(X, Y, g, st);
+    const int occ = launch_fock(X, Y, g, one);
     g.query = 0;
     if (occ < 1) return -1.0;
     int ctas[3] = {occ, occ - 1, (occ + 1) / 2};
@@ -1130,7 +1220,7 @@ static double tune_launch(int kind, int X, int Y, int part, FockGrid g, cudaStre
             double tmin = 1e30;
             for (int r = 0; r < reps + 1; r++) {   // the first run warms up
                 if (cudaMemsetAsync(g.counter, 0, sizeof(unsigned long long) * GTF_MAX_SLICES, st) != cudaSuccess ||
-                    cudaEventRecord(e0, st) != cudaSuccess || launch_fock(X, Y, g, st) < 0 ||
+                    cudaEventRecord(e0, st) != cudaSuccess || launch_fock(X, Y, g, one) < 0 ||
                     cudaEventRecord(e1, st) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess)
                     return -1.0;
                 float ms = 0.0f;
@@ -1178,7 +1268,7 @@ static int upload_basis(gtf_fock_dev *f, const gtf_basis_view_t *b)
     CK(cudaEventCreate(&f->ev1));
     CK(cudaEventCreate(&f->ev2));
     CK(cudaEventCreate(&f->ev3));
-    for (int c = 0; c <= NCLSPAIR; c++) CK(cudaEventCreate(&f->ev_cls[c]));
+    for (cudaEvent_t &e : f->ev_cls) CK(cudaEventCreate(&e));
     f->natoms = b->natoms;
     f->nshells = b->nshells;
     f->nbf = b->nbf;
@@ -1737,8 +1827,9 @@ extern "C" void gtf_fock_destroy(gtf_fock_dev_t *f)
     cudaEvent_t evs[] = {f->ev0, f->ev1, f->ev2, f->ev3};
     for (cudaEvent_t e : evs)
         if (e) cudaEventDestroy(e);
-    for (int c = 0; c <= NCLSPAIR; c++)
-        if (f->ev_cls[c]) cudaEventDestroy(f->ev_cls[c]);
+    for (cudaEvent_t e : f->ev_cls)
+        if (e) cudaEventDestroy(e);
+    f->side.give_back();
     if (f->stream) cudaStreamDestroy(f->stream);
     delete f;
 }
@@ -2030,7 +2121,7 @@ static void fill_launch(const gtf_fock_dev *f, int c, int part, const double *D,
 // builds): every part that can have work is launched, with its unit count
 // read by the kernel and its grid sized for the bound.
 static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *Fj, double *Fk,
-                        unsigned long long *counters, cudaStream_t st, int konly = 0, bool dyn = false)
+                        unsigned long long *counters, FockStreams &st, int konly = 0, bool dyn = false)
 {
     const ClassPairTask &t = f->tasks[c];
     int n = 0;
@@ -2065,6 +2156,41 @@ static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *F
         n += r;
     }
     return n;
+}
+
+// Builds of at most this many units (32 lanes each) over all launches run
+// them over several streams.  A launch of a small molecule occupies a few SMs
+// for the latency of its longest lane, and up to 62 of them (124 in mixed
+// precision) in a row add up.  Above, one launch fills the GPU: overlapping
+// tails gained at most 1.6% on C54H18 / cc-pVDZ (13.4M units) and (H2O)64 /
+// 6-31G (9.8M), and the times per class pair would no longer add up.
+#define GTF_OVERLAP_UNITS 2000000LL
+
+// All class pairs of one build; timed: events around each; may_create: the
+// side streams may be created.
+static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *Fk, unsigned long long *counters,
+                          int konly = 0, bool dyn = false, bool timed = false, bool may_create = true)
+{
+    FockStreams fs(f->stream);
+    long long units = 0;
+    int classes = 0;
+    for (const ClassPairTask &t : f->tasks) {
+        units += dyn ? t.nunits_bound : t.nunits + t.nunits32;
+        classes += t.nbra > 0 && t.nketcls > 0;
+    }
+    // 6 class pairs of s and p shells: few launches; with d shells 62
+    if (units <= GTF_OVERLAP_UNITS && (f->side.p || may_create)) CK(f->side.fork(fs, classes));
+    for (int c = 0; c < NCLSPAIR; c++) {
+        if (f->tasks[c].nbra == 0 || f->tasks[c].nketcls == 0) continue;
+        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c], fs.s[fs.next]));
+        fs.last = fs.s[fs.next];
+        const int r = launch_class(f, c, D, Fj, Fk, counters, fs, konly, dyn);
+        if (r < 0) return GTF_ERR_CUDA;
+        gtf_note_launches(r);
+        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c + 1], fs.last));
+    }
+    CK(f->side.join(fs));
+    return GTF_OK;
 }
 
 // One incremental build of density 0 (see k_delta): the change of D since
@@ -2106,13 +2232,8 @@ static int fock_compute_incremental(gtf_fock_dev *f)
     CK(cudaMemsetAsync(f->d_Fk, 0, sizeof(double) * nnc, st));
     CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, st));
     CK(cudaEventRecord(f->ev1, st));
-    for (int c = 0; c < NCLSPAIR; c++) {
-        CK(cudaEventRecord(f->ev_cls[c], st));
-        const int n = launch_class(f, c, Dc, f->d_Fj, f->d_Fk, f->d_counters, st, 0, true);
-        if (n < 0) return GTF_ERR_CUDA;
-        gtf_note_launches(n);
-    }
-    CK(cudaEventRecord(f->ev_cls[NCLSPAIR], st));
+    r = launch_classes(f, Dc, f->d_Fj, f->d_Fk, f->d_counters, 0, true, true);
+    if (r) return r;
     CK(cudaEventRecord(f->ev2, st));
     dim3 g2((nbf + 127) / 128, nbf);
     k_f_to_sph<<<g2, 128, 0, st>>>(f->d_Fj, f->d_Fk, f->d_F, f->d_J, f->d_K, f->d_sph2shell, f->d_sh_L,
@@ -2126,7 +2247,8 @@ static int fock_compute_incremental(gtf_fock_dev *f)
     CK(cudaEventElapsedTime(&eri, f->ev1, f->ev2));
     for (int c = 0; c < NCLSPAIR; c++) {
         float mc = 0.0f;
-        CK(cudaEventElapsedTime(&mc, f->ev_cls[c], f->ev_cls[c + 1]));
+        if (f->tasks[c].nbra > 0 && f->tasks[c].nketcls > 0)
+            CK(cudaEventElapsedTime(&mc, f->ev_cls[2 * c], f->ev_cls[2 * c + 1]));
         f->ms_cls[c] = mc;
     }
     f->ms_total = tot;
@@ -2219,14 +2341,8 @@ extern "C" int gtf_fock_compute(gtf_fock_dev_t *f, int numdmat)
         CK(cudaMemsetAsync(f->d_Fk, 0, sizeof(double) * nnc, st));
         CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, st));
         CK(cudaEventRecord(f->ev1, st));
-        for (int c = 0; c < NCLSPAIR; c++) {
-            ClassPairTask &t = f->tasks[c];
-            CK(cudaEventRecord(f->ev_cls[c], st));
-            (void)t;
-            const int r = launch_class(f, c, Dc, f->d_Fj, f->d_Fk, f->d_counters, st);
-            if (r < 0) return GTF_ERR_CUDA;
-            gtf_note_launches(r);
-        }
+        int r = launch_classes(f, Dc, f->d_Fj, f->d_Fk, f->d_counters, 0, false, true);
+        if (r) return r;
         if (f->nosymm) {
             const double *Dca = f->d_Da;
             if (need_tr) {
@@ -2239,11 +2355,8 @@ extern "C" int gtf_fock_compute(gtf_fock_dev_t *f, int numdmat)
             }
             CK(cudaMemsetAsync(f->d_Fka, 0, sizeof(double) * nnc, st));
             CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, st));
-            for (int c = 0; c < NCLSPAIR; c++) {
-                const int r = launch_class(f, c, Dca, f->d_Fj, f->d_Fka, f->d_counters, st, 1);
-                if (r < 0) return GTF_ERR_CUDA;
-                gtf_note_launches(r);
-            }
+            r = launch_classes(f, Dca, f->d_Fj, f->d_Fka, f->d_counters, 1);
+            if (r) return r;
         }
         if (f->nosymm == GTF_NOSYMM_REFERENCE) {
             // the reference's orientation-dependent Coulomb part: a plain
@@ -2261,13 +2374,9 @@ extern "C" int gtf_fock_compute(gtf_fock_dev_t *f, int numdmat)
             CK(cudaMemsetAsync(f->d_Fja, 0, sizeof(double) * nnc, st));
             CK(cudaMemsetAsync(f->d_Fscr, 0, sizeof(double) * nnc, st));
             CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, st));
-            for (int c = 0; c < NCLSPAIR; c++) {
-                const int r = launch_class(f, c, Dcta, f->d_Fja, f->d_Fscr, f->d_counters, st);
-                if (r < 0) return GTF_ERR_CUDA;
-                gtf_note_launches(r);
-            }
+            r = launch_classes(f, Dcta, f->d_Fja, f->d_Fscr, f->d_counters);
+            if (r) return r;
         }
-        CK(cudaEventRecord(f->ev_cls[NCLSPAIR], st));
         CK(cudaEventRecord(f->ev2, st));
         dim3 g2((nbf + 127) / 128, nbf);
         k_f_to_sph<<<g2, 128, 0, st>>>(f->d_Fj, f->d_Fk, f->d_F + nn * d, f->d_J + nn * d, f->d_K + nn * d,
@@ -2276,18 +2385,18 @@ extern "C" int gtf_fock_compute(gtf_fock_dev_t *f, int numdmat)
                                        f->nosymm == GTF_NOSYMM_REFERENCE ? f->d_Fja : nullptr);
         CK(cudaGetLastError());
         gtf_note_launches(1);
-        CK(cudaEventSynchronize(f->ev2));
+        if (d + 1 == numdmat) CK(cudaEventRecord(f->ev3, st));
+        CK(cudaEventSynchronize(d + 1 == numdmat ? f->ev3 : f->ev2));
         float ms = 0.0f;
         CK(cudaEventElapsedTime(&ms, f->ev1, f->ev2));
         eri_ms_total += ms;
         for (int c = 0; c < NCLSPAIR; c++) {
             float mc = 0.0f;
-            CK(cudaEventElapsedTime(&mc, f->ev_cls[c], f->ev_cls[c + 1]));
+            if (f->tasks[c].nbra > 0 && f->tasks[c].nketcls > 0)
+                CK(cudaEventElapsedTime(&mc, f->ev_cls[2 * c], f->ev_cls[2 * c + 1]));
             f->ms_cls[c] = (d == 0 ? 0.0 : f->ms_cls[c]) + mc;
         }
     }
-    CK(cudaEventRecord(f->ev3, st));
-    CK(cudaEventSynchronize(f->ev3));
     float tot = 0.0f;
     CK(cudaEventElapsedTime(&tot, f->ev0, f->ev3));
     f->ms_total = tot;
@@ -2618,8 +2727,8 @@ extern "C" int gtf_fock_compute_fixed(gtf_fock_dev_t *f, const double *dev_D, do
     CK(cudaMemsetAsync(Fj, 0, sizeof(double) * nnc, st));
     CK(cudaMemsetAsync(Fk, 0, sizeof(double) * nnc, st));
     CK(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, st));
-    for (int c = 0; c < NCLSPAIR; c++)
-        if (launch_class(f, c, Duse, Fj, Fk, counters, st) < 0) return GTF_ERR_CUDA;
+    r = launch_classes(f, Duse, Fj, Fk, counters, 0, false, false, false);
+    if (r) return r;
     dim3 g2((nbf + 127) / 128, nbf);
     k_f_to_sph<<<g2, 128, 0, st>>>(Fj, Fk, dev_F, J, K, f->d_sph2shell, f->d_sh_L, f->d_f_start, f->d_fc_start,
                                    nbf, nbfc, f->pure);
@@ -2753,6 +2862,7 @@ struct gtf_fock_batch {
     int npdesc;
     size_t maxnn;
     std::vector<const long long *> solo_tot[NCLSPAIR][2];
+    ForkJoin side;
 };
 
 // A molecule whose units in one launch reach this many (32 quartets each)
@@ -2803,6 +2913,7 @@ extern "C" void gtf_fock_batch_destroy(gtf_fock_batch_t *b)
             gtf_dfree(b->d_desc[c][p], st);
             gtf_dfree(b->d_prefix[c][p], st);
         }
+    b->side.give_back();
     delete b;
 }
 
@@ -3063,6 +3174,14 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
     }
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned long long) * (size_t)b->ncounter_blocks * GTF_MAX_SLICES,
                        st));
+    FockStreams fs(st);
+    long long units = 0;
+    for (int c = 0; c < NCLSPAIR; c++)
+        for (int p = 0; p < 2; p++) {
+            units += b->total[c][p];
+            for (long long n : b->solo_units[c][p]) units += n;
+        }
+    if (units <= GTF_OVERLAP_UNITS) CK(b->side.fork(fs, GTF_FOCK_STREAMS));
     for (int c = 0; c < NCLSPAIR; c++) {
         const ClassPairTask &t0 = b->eng[0]->tasks[c];
         for (int p = 0; p < 2; p++) {
@@ -3077,7 +3196,7 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
                 g.nsm = b->nsm;
                 g.fp32 = p;
                 tune_apply(0, t0.X, t0.Y, p, g);
-                const int r = launch_fock(t0.X, t0.Y, g, st);
+                const int r = launch_fock(t0.X, t0.Y, g, fs);
                 if (r < 0) {
                     snprintf(g_errbuf, sizeof(g_errbuf), "Fock launch for class pair %d part %d failed: %s", c, p,
                              cudaGetErrorString(cudaGetLastError()));
@@ -3098,7 +3217,7 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
             g.nsm = b->nsm;
             g.fp32 = p;
             tune_apply(1, t0.X, t0.Y, p, g);
-            const int r = launch_fock(t0.X, t0.Y, g, st);
+            const int r = launch_fock(t0.X, t0.Y, g, fs);
             if (r < 0) {
                 snprintf(g_errbuf, sizeof(g_errbuf), "batched Fock launch for class pair %d part %d failed: %s", c, p,
                          cudaGetErrorString(cudaGetLastError()));
@@ -3107,6 +3226,7 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
             launches += r;
         }
     }
+    CK(b->side.join(fs));
     {
         dim3 g((b->maxn + 127) / 128, b->maxn < 1024 ? b->maxn : 1024, b->M);
         k_b_post<<<g, 128, 0, st>>>(b->d_xf);

@@ -2,7 +2,7 @@
 // angular class pairs (split for parallel compilation).
 #include "fock_kernel.cuh"
 
-extern "C" int gtf_fock_group_3(int la, int lb, int lc, int ld, const FockGrid &g, cudaStream_t st)
+extern "C" int gtf_fock_group_3(int la, int lb, int lc, int ld, const FockGrid &g, FockStreams &st)
 {
     FOCK_GROUP_CASE(2,2,1,1)
     FOCK_GROUP_CASE(2,2,2,0)

@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "gtf_cuda.h"
 #include "gtf_dev.cuh"
 
@@ -275,6 +277,22 @@ __global__ void __launch_bounds__(FOCK_THREADS,
     }
 }
 
+// Streams the launches of a build are dealt out to in turn (n == 1: all in
+// order on one stream).
+#define GTF_FOCK_STREAMS 8
+struct FockStreams {
+    cudaStream_t s[GTF_FOCK_STREAMS];
+    int n, next;
+    cudaStream_t last;   // stream of the latest launch
+    explicit FockStreams(cudaStream_t st) : n(1), next(0), last(st) { s[0] = st; }
+    cudaStream_t take()
+    {
+        last = s[next];
+        next = next + 1 < n ? next + 1 : 0;
+        return last;
+    }
+};
+
 // Number of slice launches of a class pair; g.counter points at that many
 // zeroed counters.
 __host__ __device__ constexpr int fock_nslices(int LA, int LB, int LC, int LD, int fp32)
@@ -285,22 +303,27 @@ __host__ __device__ constexpr int fock_nslices(int LA, int LB, int LC, int LD, i
 #define GTF_MAX_SLICES 64
 
 template <int LA, int LB, int LC, int LD, typename R, int CD0>
-int launch_fock_slices(const FockGrid &g, cudaStream_t st, int slice)
+int launch_fock_slices(const FockGrid &g, FockStreams &st, int slice)
 {
     constexpr int NCD = ncart(LC) * ncart(LD);
     if constexpr (CD0 < NCD) {
         constexpr int S = fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
         auto k = g.nmol > 1 ? k_fock<LA, LB, LC, LD, R, CD0, true> : k_fock<LA, LB, LC, LD, R, CD0, false>;
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k, FOCK_THREADS, 0);
-        if (per_sm < 1) per_sm = 1;
+        // the same on every device this code runs on (sm_100a): asked once
+        static std::atomic<int> occ[2];
+        int per_sm = occ[g.nmol > 1].load(std::memory_order_relaxed);
+        if (per_sm == 0) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)k, FOCK_THREADS, 0);
+            if (per_sm < 1) per_sm = 1;
+            occ[g.nmol > 1].store(per_sm, std::memory_order_relaxed);
+        }
         if (g.query) return per_sm;
         if (g.ctas_per_sm > 0 && g.ctas_per_sm < per_sm) per_sm = g.ctas_per_sm;
         long long want = (g.nunits + (FOCK_THREADS / 32) - 1) / (FOCK_THREADS / 32);
         long long grid = (long long)g.nsm * per_sm;
         if (want < grid) grid = want;
         if (grid < 1) grid = 1;
-        k<<<(unsigned)grid, FOCK_THREADS, 0, st>>>(g, g.counter + slice);
+        k<<<(unsigned)grid, FOCK_THREADS, 0, st.take()>>>(g, g.counter + slice);
         if (cudaGetLastError() != cudaSuccess) return -1;
         const int r = launch_fock_slices<LA, LB, LC, LD, R, CD0 + S>(g, st, slice + 1);
         return r < 0 ? r : r + 1;
@@ -311,7 +334,7 @@ int launch_fock_slices(const FockGrid &g, cudaStream_t st, int slice)
 
 // returns the number of kernels launched, or -1 on a launch error
 template <int LA, int LB, int LC, int LD, typename R>
-int launch_fock_t(const FockGrid &g, cudaStream_t st)
+int launch_fock_t(const FockGrid &g, FockStreams &st)
 {
     static_assert(fock_nslices(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0) <= GTF_MAX_SLICES, "slice counters");
     return launch_fock_slices<LA, LB, LC, LD, R, 0>(g, st, 0);
