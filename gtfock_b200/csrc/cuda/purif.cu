@@ -49,7 +49,7 @@ struct gtf_purif_dev {
     cublasHandle_t blas;      // leased for the duration of one call (BlasLease)
     double *S, *X, *D, *D2, *D3, *F, *W, *W2;
     double *vecs, *Fvecs;
-    double *part;     // [RED_BLOCKS * 16] block partials
+    double *part;     // [part_len(n)] block partials
     double *scal;     // device scalars
     double *h_scal;   // pinned mirror
     double *E;        // this iteration's DIIS error vector, before it enters its slot
@@ -61,6 +61,15 @@ struct gtf_purif_dev {
     gtf_bf16x3_t *bx;
     int it_bf16, it_fp64;
 };
+
+#define GERSH_COLS 32
+#define GERSH_ROWS 8
+// block partials: 16 per reduction block, or 3 per block of the Gershgorin pass
+static size_t part_len(int n)
+{
+    const size_t a = (size_t)RED_BLOCKS * 16, b = 3 * (size_t)((n + GERSH_COLS - 1) / GERSH_COLS);
+    return a > b ? a : b;
+}
 
 // row-major C = A B^T (pdgemm3D_2) and C = A B, via column-major cuBLAS
 static int gemm_abt(gtf_purif_dev *p, const double *A, const double *B, double *C)
@@ -77,53 +86,71 @@ static int gemm_ab(gtf_purif_dev *p, const double *A, const double *B, double *C
     return GTF_OK;
 }
 
+// sums over the 32 lanes, the same total in every lane
+__device__ __forceinline__ double warp_sum(double v)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
 // per column i: Gershgorin interval [diag - off, diag + off], off = sum_j |F[j][i]| - |diag|
-// (pscf/purif.c:309-322); block partials of min, max and the trace
+// (pscf/purif.c:309-322); block partials of min, max and the trace.  A block
+// takes 32 columns, its 8 rows of threads every 8th matrix row: one thread
+// walking a whole column kept 4 blocks busy for 360 us at 846 functions.
+static_assert(GERSH_COLS * GERSH_ROWS == RED_THREADS, "block shape");
 __global__ void k_gersh(const double *__restrict__ F, int n, double *__restrict__ part)
 {
-    __shared__ double smin[RED_THREADS], smax[RED_THREADS], str[RED_THREADS];
-    double lmin = DBL_MAX, lmax = -DBL_MAX, ltr = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        double off = 0.0, dg = 0.0;
-        for (int j = 0; j < n; j++) {
-            const double v = F[(size_t)j * n + i];
-            off += fabs(v);
-            if (j == i) dg = v;
-        }
-        off -= fabs(dg);
-        lmin = fmin(lmin, dg - off);
-        lmax = fmax(lmax, dg + off);
-        ltr += dg;
+    __shared__ double soff[GERSH_ROWS][GERSH_COLS];
+    const int c = threadIdx.x % GERSH_COLS, r = threadIdx.x / GERSH_COLS, i = blockIdx.x * GERSH_COLS + c;
+    double off = 0.0;
+    if (i < n) {
+#pragma unroll 4
+        for (int j = r; j < n; j += GERSH_ROWS) off += fabs(F[(size_t)j * n + i]);
     }
-    smin[threadIdx.x] = lmin;
-    smax[threadIdx.x] = lmax;
-    str[threadIdx.x] = ltr;
+    soff[r][c] = off;
     __syncthreads();
-    for (int s = RED_THREADS / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            smin[threadIdx.x] = fmin(smin[threadIdx.x], smin[threadIdx.x + s]);
-            smax[threadIdx.x] = fmax(smax[threadIdx.x], smax[threadIdx.x + s]);
-            str[threadIdx.x] += str[threadIdx.x + s];
-        }
-        __syncthreads();
+    if (r != 0) return;
+    double lmin = DBL_MAX, lmax = -DBL_MAX, ltr = 0.0;
+    if (i < n) {
+        off = 0.0;
+#pragma unroll
+        for (int k = 0; k < GERSH_ROWS; k++) off += soff[k][c];
+        const double dg = F[(size_t)i * n + i];
+        off -= fabs(dg);
+        lmin = dg - off;
+        lmax = dg + off;
+        ltr = dg;
     }
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = smin[0];
-        part[3 * blockIdx.x + 1] = smax[0];
-        part[3 * blockIdx.x + 2] = str[0];
+    ltr = warp_sum(ltr);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        lmin = fmin(lmin, __shfl_xor_sync(0xffffffffu, lmin, o));
+        lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+    }
+    if (c == 0) {
+        part[3 * blockIdx.x] = lmin;
+        part[3 * blockIdx.x + 1] = lmax;
+        part[3 * blockIdx.x + 2] = ltr;
     }
 }
 
 // scal[0] = -lambda/n, scal[1] = lambda mu_bar / n + nocc / n (pscf/purif.c:355-373)
 __global__ void k_purif_init(const double *__restrict__ part, int nblk, int n, int nocc, double *scal)
 {
-    if (threadIdx.x != 0) return;
     double hmin = DBL_MAX, hmax = -DBL_MAX, trF = 0.0;
-    for (int b = 0; b < nblk; b++) {
+    for (int b = threadIdx.x; b < nblk; b += 32) {
         hmin = fmin(hmin, part[3 * b]);
         hmax = fmax(hmax, part[3 * b + 1]);
         trF += part[3 * b + 2];
     }
+    trF = warp_sum(trF);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        hmin = fmin(hmin, __shfl_xor_sync(0xffffffffu, hmin, o));
+        hmax = fmax(hmax, __shfl_xor_sync(0xffffffffu, hmax, o));
+    }
+    if (threadIdx.x != 0) return;
     const double mu_bar = trF / (double)n;
     const double lambda = fmin((double)nocc / (hmax - mu_bar), (double)(n - nocc) / (mu_bar - hmin));
     scal[0] = -lambda / n;
@@ -147,9 +174,10 @@ __global__ void k_purif_d0(const double *__restrict__ F, double *__restrict__ D,
 __global__ void k_purif_stats(const double *__restrict__ D, const double *__restrict__ D2,
                               const double *__restrict__ D3, int n, double *__restrict__ part)
 {
-    __shared__ double s0[RED_THREADS], s1[RED_THREADS], s2[RED_THREADS];
+    __shared__ double sh[3][RED_THREADS / 32];
     const size_t nn = (size_t)n * n;
     double e = 0.0, t = 0.0, t2 = 0.0;
+#pragma unroll 4
     for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < nn; k += (size_t)gridDim.x * blockDim.x) {
         const double d = D[k] - D2[k];
         e += d * d;
@@ -159,22 +187,20 @@ __global__ void k_purif_stats(const double *__restrict__ D, const double *__rest
         t += D2[k] - D3[k];
         t2 += D[k] - D2[k];
     }
-    s0[threadIdx.x] = e;
-    s1[threadIdx.x] = t;
-    s2[threadIdx.x] = t2;
-    __syncthreads();
-    for (int s = RED_THREADS / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            s0[threadIdx.x] += s0[threadIdx.x + s];
-            s1[threadIdx.x] += s1[threadIdx.x + s];
-            s2[threadIdx.x] += s2[threadIdx.x + s];
-        }
-        __syncthreads();
+    e = warp_sum(e);
+    t = warp_sum(t);
+    t2 = warp_sum(t2);
+    if ((threadIdx.x & 31) == 0) {
+        sh[0][threadIdx.x >> 5] = e;
+        sh[1][threadIdx.x >> 5] = t;
+        sh[2][threadIdx.x >> 5] = t2;
     }
-    if (threadIdx.x == 0) {
-        part[3 * blockIdx.x] = s0[0];
-        part[3 * blockIdx.x + 1] = s1[0];
-        part[3 * blockIdx.x + 2] = s2[0];
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        double v = 0.0;
+#pragma unroll
+        for (int w = 0; w < RED_THREADS / 32; w++) v += sh[threadIdx.x][w];
+        part[3 * blockIdx.x + threadIdx.x] = v;
     }
 }
 
@@ -200,20 +226,25 @@ __global__ void k_purif_stats(const double *__restrict__ D, const double *__rest
 #define PURIF_TOL 1e-11
 #define PURIF_STALL 8
 #define PURIF_FLOOR 1e-8
+// One warp: a single thread reading the 148 partials took 20 us of a step.
 __global__ void k_purif_finish(const double *__restrict__ part, int nblk, double *scal)
 {
-    if (threadIdx.x != 0) return;
     const double nan = __longlong_as_double(0x7ff8000000000000LL);
     if (scal[8] != 0.0) {
-        scal[7] = nan;   // stopped: no update
+        if (threadIdx.x == 0) scal[7] = nan;   // stopped: no update
         return;
     }
     double e = 0.0, t = 0.0, t2 = 0.0;
-    for (int b = 0; b < nblk; b++) {
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nblk; b += 32) {
         e += part[3 * b];
         t += part[3 * b + 1];
         t2 += part[3 * b + 2];
     }
+    e = warp_sum(e);
+    t = warp_sum(t);
+    t2 = warp_sum(t2);
+    if (threadIdx.x != 0) return;
     const double c = t / t2;
     const bool ok = isfinite(c) && c >= PURIF_C_LO && c <= PURIF_C_HI;
     scal[6] = ok ? sqrt(e) : 0.0;
@@ -310,6 +341,7 @@ __global__ void k_diis_solve(const double *__restrict__ part, DiisState *ds)
     const int lane = threadIdx.x;
     if (lane < ds->len) {
         double v = 0.0;
+#pragma unroll 8
         for (int bk = 0; bk < RED_BLOCKS; bk++) v += part[bk * PUR_MAX_DIIS + lane];
         dots[lane] = v;
     }
@@ -353,7 +385,7 @@ extern "C" int gtf_purif_create(int nbf, int nocc, void *stream, gtf_purif_dev_t
     for (double **b : bufs) CKP(gtf_dmalloc((void **)b, sizeof(double) * nn, p->st));
     CKP(gtf_dmalloc((void **)&p->vecs, sizeof(double) * nn * PUR_MAX_DIIS, p->st));
     CKP(gtf_dmalloc((void **)&p->Fvecs, sizeof(double) * nn * PUR_MAX_DIIS, p->st));
-    CKP(gtf_dmalloc((void **)&p->part, sizeof(double) * RED_BLOCKS * 16, p->st));
+    CKP(gtf_dmalloc((void **)&p->part, sizeof(double) * part_len(p->n), p->st));
     CKP(gtf_dmalloc((void **)&p->scal, sizeof(double) * 16, p->st));
     p->h_scal = (double *)gtf_pinned_alloc(sizeof(double) * 16);
     if (!p->h_scal) return GTF_ERR_ALLOC;
@@ -434,8 +466,9 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
     const unsigned ge = (unsigned)((nn + 255) / 256);
     cudaStream_t st = p->st;
     CKP(cudaEventRecord(p->e0, st));
-    k_gersh<<<RED_BLOCKS, RED_THREADS, 0, st>>>(F_dev, n, p->part);
-    k_purif_init<<<1, 32, 0, st>>>(p->part, RED_BLOCKS, n, p->nocc, p->scal);
+    const int gb = (n + GERSH_COLS - 1) / GERSH_COLS;
+    k_gersh<<<gb, RED_THREADS, 0, st>>>(F_dev, n, p->part);
+    k_purif_init<<<1, 32, 0, st>>>(p->part, gb, n, p->nocc, p->scal);
     k_purif_d0<<<ge, 256, 0, st>>>(F_dev, p->D, n, p->scal);
     CKP(cudaGetLastError());
     gtf_note_launches(3);
