@@ -72,6 +72,7 @@ static const int k_cls_la[NCLS] = {0, 1, 1, 2, 2, 2};
 static const int k_cls_lb[NCLS] = {0, 0, 1, 0, 1, 2};
 
 struct UnitTask;
+#define UNIT_TOTALS 5   // totals per task (k_unit_totals)
 
 static inline double __longlong_as_double_host(unsigned long long b)
 {
@@ -266,7 +267,7 @@ struct gtf_fock_dev {
     double incr_tau;
     double *d_Dprev, *d_Dd;
     DynState *d_dyn;
-    unsigned long long *d_unit_tot;  // [NCLSPAIR][3] quartets, FP32 quartets, unit bound (build_units)
+    unsigned long long *d_unit_tot;  // [NCLSPAIR][UNIT_TOTALS] (k_unit_totals)
     // the task-list arrays hold an incremental build's lists (rebuilt from
     // the static thresholds before a plain build uses them)
     int lists_dyn;
@@ -739,14 +740,22 @@ __global__ void k_build_pairs(const int *__restrict__ idx, const int *__restrict
 // Primitive pairs of each listed shell pair, compacted and sorted: pairs
 // whose prefactor |K| is below GTF_PRIM_EPS are dropped (their contribution
 // to any integral is below ~1e-15 Hartree), the rest are stored in descending
-// |K| so that the quartet loop can stop once |K_ab K_cd| < GTF_PRIMQ_EPS.
-// pairs[s].n becomes the kept count (possibly 0); the slot keeps its size.
-// Records are {p, K, Px, Py, Pz, 1/(2p)} (PPRec).
-__global__ void k_fill_primpairs(PairRec *__restrict__ pairs, const int *__restrict__ idx,
-                                 const int *__restrict__ shellid, const int *__restrict__ shellrid,
-                                 const int *__restrict__ pair_off, BasisDev b, int npairs, double *pp)
+// |K| (equal ones in the order of the shells' primitives) so that the quartet
+// loop can stop once |K_ab K_cd| < GTF_PRIMQ_EPS.  pairs[s].n becomes the
+// kept count (possibly 0); the slot keeps its size.  Records are {p, K, Px,
+// Py, Pz, 1/(2p)} (PPRec).  A warp per shell pair: the |K| of its primitive
+// pairs go to shared memory, and each kept one is written at its rank among
+// them (one thread sorting up to 64 records in global memory by insertion
+// took 1.5 ms for C12H26 / cc-pVDZ).
+#define FILL_WARPS 4
+#define FILL_MAX 256   // primitive pairs kept in shared memory; the rest are evaluated again for each rank
+__global__ void __launch_bounds__(32 * FILL_WARPS)
+    k_fill_primpairs(PairRec *__restrict__ pairs, const int *__restrict__ idx, const int *__restrict__ shellid,
+                     const int *__restrict__ shellrid, const int *__restrict__ pair_off, BasisDev b, int npairs,
+                     double *__restrict__ pp)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double sh[FILL_WARPS][FILL_MAX];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, s = blockIdx.x * FILL_WARPS + w;
     if (s >= npairs) return;
     const int k = idx[s];
     const int M = shellrid[k], N = shellid[k];
@@ -756,35 +765,42 @@ __global__ void k_fill_primpairs(PairRec *__restrict__ pairs, const int *__restr
     const double Ax = b.sh_xyz[3 * a], Ay = b.sh_xyz[3 * a + 1], Az = b.sh_xyz[3 * a + 2];
     const double Bx = b.sh_xyz[3 * bb], By = b.sh_xyz[3 * bb + 1], Bz = b.sh_xyz[3 * bb + 2];
     const double r2 = (Ax - Bx) * (Ax - Bx) + (Ay - By) * (Ay - By) + (Az - Bz) * (Az - Bz);
-    const int na = b.sh_nprim[a], nb = b.sh_nprim[bb];
+    const int nb = b.sh_nprim[bb], n = b.sh_nprim[a] * nb;
     const int pa = b.sh_pstart[a], pb = b.sh_pstart[bb];
+    auto abs_k = [&](int q) {
+        double p;
+        return fabs(prim_pair_K(b, pa, pb, q / nb, q % nb, r2, p));
+    };
+    for (int q = lane; q < n && q < FILL_MAX; q += 32) sh[w][q] = abs_k(q);
+    __syncwarp();
     constexpr int W = 2 * GTF_PPREC_D2;
     int kept = 0;
-    for (int i = 0; i < na; i++) {
-        for (int j = 0; j < nb; j++) {
-            double p;
-            const double K = prim_pair_K(b, pa, pb, i, j, r2, p);
-            if (fabs(K) < GTF_PRIM_EPS) continue;
-            const double al = b.alpha[pa + i], be = b.alpha[pb + j], ip = 1.0 / p;
-            // insertion into the descending-|K| list of the kept pairs
-            int o = kept;
-            while (o > 0 && fabs(pp[W * ((size_t)off + o - 1) + 1]) < fabs(K)) {
-                const size_t src = W * ((size_t)off + o - 1);
-                for (int f = 0; f < W; f++) pp[src + W + f] = pp[src + f];
-                o--;
-            }
-            double *d = pp + W * ((size_t)off + o);
-            d[0] = p;
-            d[1] = K;
-            d[2] = (al * Ax + be * Bx) * ip;
-            d[3] = (al * Ay + be * By) * ip;
-            d[4] = (al * Az + be * Bz) * ip;
-            d[5] = 0.5 * ip;
-            kept++;
+    for (int q = lane; q < n; q += 32) {
+        const int i = q / nb, j = q % nb;
+        double p;
+        const double K = prim_pair_K(b, pa, pb, i, j, r2, p);
+        const double v = fabs(K);
+        if (v < GTF_PRIM_EPS) continue;
+        kept++;
+        int o = 0;
+        for (int t = 0; t < n; t++) {
+            const double u = t < FILL_MAX ? sh[w][t] : abs_k(t);
+            if (u >= GTF_PRIM_EPS && (u > v || (u == v && t < q))) o++;
         }
+        const double al = b.alpha[pa + i], be = b.alpha[pb + j], ip = 1.0 / p;
+        double *d = pp + W * ((size_t)off + o);
+        d[0] = p;
+        d[1] = K;
+        d[2] = (al * Ax + be * Bx) * ip;
+        d[3] = (al * Ay + be * By) * ip;
+        d[4] = (al * Az + be * Bz) * ip;
+        d[5] = 0.5 * ip;
     }
-    pairs[s].off = off;
-    pairs[s].n = kept;
+    kept = __reduce_add_sync(GTF_FULL_MASK, kept);
+    if (lane == 0) {
+        pairs[s].off = off;
+        pairs[s].n = kept;
+    }
 }
 
 // FP32 records of the kept primitive pairs: centre relative to the pair's
@@ -792,11 +808,11 @@ __global__ void k_fill_primpairs(PairRec *__restrict__ pairs, const int *__restr
 __global__ void k_fill_pp32(const PairRec *__restrict__ pairs, int npairs, const double *__restrict__ pp,
                             float *__restrict__ pp32)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    const int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 3;   // 8 threads per pair
     if (s >= npairs) return;
     const PairRec r = pairs[s];
     constexpr int W = 2 * GTF_PPREC_D2;
-    for (int i = 0; i < r.n; i++) {
+    for (int i = threadIdx.x & 7; i < r.n; i += 8) {
         const double *d = pp + W * ((size_t)r.off + i);
         float *o = pp32 + 8 * ((size_t)r.off + i);
         o[0] = (float)d[0];
@@ -1372,7 +1388,7 @@ static int make_unit_tasks(gtf_fock_dev *f)
     DALLOC(f->d_ut_static, nt);
     DALLOC(f->d_ut_dyn, nt);
     DALLOC(f->d_dyn, 1);
-    DALLOC(f->d_unit_tot, 3 * NCLSPAIR);
+    DALLOC(f->d_unit_tot, UNIT_TOTALS * NCLSPAIR);
     std::vector<UnitTask> dyn(f->h_ut);
     for (auto &u : dyn) u.dyn = f->d_dyn;
     if (nt) CK(cudaMemcpyAsync(f->d_ut_dyn, dyn.data(), sizeof(UnitTask) * nt, cudaMemcpyHostToDevice, f->stream));
@@ -1383,21 +1399,22 @@ static int make_unit_tasks(gtf_fock_dev *f)
 
 static int shard_bounds(gtf_fock_dev *f, int c, const std::vector<int> &nk, const std::vector<int> &n64);
 
-// Totals of one class pair's (bra, segment) ket counts: quartets, FP32
-// quartets and the bound on a launch's units (sum over bras of the units of
-// all non-empty segments).  64-bit integer sums: exact whatever the order.
-__global__ void k_unit_totals(const int *__restrict__ nk, const int *__restrict__ n64,
-                              const int *__restrict__ cum64, const int *__restrict__ cum32, int nbra,
-                              unsigned long long *__restrict__ out)
+// Totals of every task's (bra, segment) ket counts (task blockIdx.y): quartets,
+// FP32 quartets, the bound on a launch's units (sum over bras of the units of
+// all non-empty segments) and the units of the FP64 and the FP32 launch.
+// 64-bit integer sums: exact whatever the order.
+__global__ void k_unit_totals(const UnitTask *__restrict__ tasks, unsigned long long *__restrict__ out)
 {
+    const UnitTask &t = tasks[blockIdx.y];
+    out += UNIT_TOTALS * blockIdx.y;
     unsigned long long q = 0, q32 = 0, bound = 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nbra; i += gridDim.x * blockDim.x) {
-        const long long all = (long long)cum64[i * GTF_CUM + GTF_NBKT] + cum32[i * GTF_CUM + GTF_NBKT];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.nbra; i += gridDim.x * blockDim.x) {
+        const long long all = (long long)t.cum64[i * GTF_CUM + GTF_NBKT] + t.cum32[i * GTF_CUM + GTF_NBKT];
 #pragma unroll
         for (int b = 0; b < GTF_NBKT; b++) {
             const int k = i * GTF_NBKT + b;
-            q += (unsigned long long)nk[k];
-            q32 += (unsigned long long)(nk[k] - n64[k]);
+            q += (unsigned long long)t.nket[k];
+            q32 += (unsigned long long)(t.nket[k] - t.n64[k]);
         }
         bound += (unsigned long long)((all + 31) / 32);
     }
@@ -1411,6 +1428,10 @@ __global__ void k_unit_totals(const int *__restrict__ nk, const int *__restrict_
         atomicAdd(out, q);
         atomicAdd(out + 1, q32);
         atomicAdd(out + 2, bound);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        out[3] = (unsigned long long)t.up64[t.nbra];
+        out[4] = (unsigned long long)t.up32[t.nbra];
     }
 }
 
@@ -1441,38 +1462,34 @@ static int build_units(gtf_fock_dev *f)
     // the per-(bra, segment) counts come to the host only for the shard split
     const bool sharded = f->nshards > 1;
     std::vector<std::vector<int>> nk(NCLSPAIR), n64(NCLSPAIR);
-    unsigned long long tot[3 * NCLSPAIR];
+    unsigned long long tot[UNIT_TOTALS * NCLSPAIR];
     CK(cudaMemsetAsync(f->d_unit_tot, 0, sizeof(tot), st));
-    int nl = 0;
-    for (int c = 0; c < NCLSPAIR; c++) {
+    k_unit_totals<<<dim3(16, nt), 256, 0, st>>>(f->d_ut_static, f->d_unit_tot);
+    CK(cudaGetLastError());
+    gtf_note_launches(1);
+    for (int c = 0; c < NCLSPAIR && sharded; c++) {
         ClassPairTask &t = f->tasks[c];
         if (t.nbra == 0 || t.nketcls == 0) continue;
         const int nidx = t.nbra * GTF_NBKT;
-        int g = (t.nbra + 255) / 256;
-        if (g > 4 * f->nsm) g = 4 * f->nsm;
-        k_unit_totals<<<g, 256, 0, st>>>(t.d_nket, t.d_n64, t.d_cum64, t.d_cum32, t.nbra, f->d_unit_tot + 3 * c);
-        CK(cudaGetLastError());
-        nl++;
-        CK(cudaMemcpyAsync(&t.nunits, t.d_unit_prefix + t.nbra, sizeof(long long), cudaMemcpyDeviceToHost, st));
-        CK(cudaMemcpyAsync(&t.nunits32, t.d_unit_prefix32 + t.nbra, sizeof(long long), cudaMemcpyDeviceToHost, st));
-        if (sharded) {
-            nk[c].resize(nidx);
-            n64[c].resize(nidx);
-            CK(cudaMemcpyAsync(nk[c].data(), t.d_nket, sizeof(int) * nidx, cudaMemcpyDeviceToHost, st));
-            CK(cudaMemcpyAsync(n64[c].data(), t.d_n64, sizeof(int) * nidx, cudaMemcpyDeviceToHost, st));
-        }
+        nk[c].resize(nidx);
+        n64[c].resize(nidx);
+        CK(cudaMemcpyAsync(nk[c].data(), t.d_nket, sizeof(int) * nidx, cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(n64[c].data(), t.d_n64, sizeof(int) * nidx, cudaMemcpyDeviceToHost, st));
     }
-    gtf_note_launches(nl);
     CK(cudaMemcpyAsync(tot, f->d_unit_tot, sizeof(tot), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    const unsigned long long *q = tot;   // in the order of the tasks
     for (int c = 0; c < NCLSPAIR; c++) {
         ClassPairTask &t = f->tasks[c];
         if (t.nbra == 0 || t.nketcls == 0) continue;
-        t.nquart = (double)tot[3 * c];
-        t.nquart32 = (double)tot[3 * c + 1];
+        t.nquart = (double)q[0];
+        t.nquart32 = (double)q[1];
         // thresholds at or above tol2 select a subset of these kets, in one
         // launch or split between two (one more unit per bra at most)
-        t.nunits_bound = (long long)tot[3 * c + 2] + t.nbra;
+        t.nunits_bound = (long long)q[2] + t.nbra;
+        t.nunits = (long long)q[3];
+        t.nunits32 = (long long)q[4];
+        q += UNIT_TOTALS;
     }
     // the units of this engine's shard (all of them when not sharded)
     f->shard_work = 0.0;
@@ -1700,10 +1717,10 @@ extern "C" int gtf_fock_create(const gtf_basis_view_t *b, double tolscr, int max
     DALLOC(f->d_pp, 2 * GTF_PPREC_D2 * (size_t)(npp > 0 ? npp : 1));
     DALLOC(f->d_pp32, 8 * (size_t)(npp > 0 ? npp : 1));
     if (nnz > 0) {
-        k_fill_primpairs<<<gp, 256, 0, st>>>(f->d_pairs, d_idx, f->d_shellid, f->d_shellrid, d_pair_off, bd,
-                                             nnz, f->d_pp);
+        k_fill_primpairs<<<(nnz + FILL_WARPS - 1) / FILL_WARPS, 32 * FILL_WARPS, 0, st>>>(
+            f->d_pairs, d_idx, f->d_shellid, f->d_shellrid, d_pair_off, bd, nnz, f->d_pp);
         CK(cudaGetLastError());
-        k_fill_pp32<<<gp, 256, 0, st>>>(f->d_pairs, nnz, f->d_pp, f->d_pp32);
+        k_fill_pp32<<<(nnz + 31) / 32, 256, 0, st>>>(f->d_pairs, nnz, f->d_pp, f->d_pp32);
         CK(cudaGetLastError());
     }
     // class and segment starts from the sorted keys (class * 16 + bucket)
