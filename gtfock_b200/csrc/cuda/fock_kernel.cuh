@@ -142,10 +142,19 @@ __host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD
     return nq <= 3 ? 6 : nq <= 9 ? 4 : nq <= 27 ? 3 : 2;
 }
 
+//
+// A launch with many units per SM runs one block of fock_max_threads on each,
+// so that the SM holds one copy of the Rys table (13 to 49 KB) and the rest
+// of its 228 KB caches the gathers of D and of the primitive records; small
+// launches spread blocks of FOCK_THREADS over the SMs.  The registers per
+// thread are the same.
+__host__ __device__ constexpr int fock_max_threads(int LA, int LB, int LC, int LD, int fp32)
+{
+    return FOCK_THREADS * fock_min_blocks(LA, LB, LC, LD, fock_slice(LA, LB, LC, LD, fp32));
+}
+
 template <int LA, int LB, int LC, int LD, typename R, int CD0, bool BATCH>
-__global__ void __launch_bounds__(FOCK_THREADS,
-                                  fock_min_blocks(LA, LB, LC, LD,
-                                                  fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0)))
+__global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0), 1)
     k_fock(const FockGrid g, unsigned long long *counter)
 {
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
@@ -162,7 +171,7 @@ __global__ void __launch_bounds__(FOCK_THREADS,
     // batched launches: per-warp slots for the claimed range of units and the
     // molecule of the current unit, so that neither holds registers across
     // the integral loops
-    constexpr int NW = FOCK_THREADS / 32;
+    constexpr int NW = fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0) / 32;
     __shared__ unsigned long long s_claim[BATCH ? 2 * NW : 1];
     __shared__ int s_mol[BATCH ? NW : 1];
     const int wib = threadIdx.x >> 5;
@@ -277,6 +286,9 @@ __global__ void __launch_bounds__(FOCK_THREADS,
     }
 }
 
+// Units per resident warp from which a launch uses one large block per SM.
+#define GTF_BIG_ROUNDS 4
+
 // Streams the launches of a build are dealt out to in turn (n == 1: all in
 // order on one stream).
 #define GTF_FOCK_STREAMS 8
@@ -318,12 +330,19 @@ int launch_fock_slices(const FockGrid &g, FockStreams &st, int slice)
             occ[g.nmol > 1].store(per_sm, std::memory_order_relaxed);
         }
         if (g.query) return per_sm;
-        if (g.ctas_per_sm > 0 && g.ctas_per_sm < per_sm) per_sm = g.ctas_per_sm;
-        long long want = (g.nunits + (FOCK_THREADS / 32) - 1) / (FOCK_THREADS / 32);
+        constexpr int BIG = fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
+        int threads = FOCK_THREADS;
+        if (g.ctas_per_sm > 0 && g.ctas_per_sm < per_sm) {
+            per_sm = g.ctas_per_sm;
+        } else if (g.nunits >= (long long)g.nsm * (BIG / 32) * GTF_BIG_ROUNDS) {
+            threads = BIG;
+            per_sm = 1;
+        }
+        long long want = (g.nunits + threads / 32 - 1) / (threads / 32);
         long long grid = (long long)g.nsm * per_sm;
         if (want < grid) grid = want;
         if (grid < 1) grid = 1;
-        k<<<(unsigned)grid, FOCK_THREADS, 0, st.take()>>>(g, g.counter + slice);
+        k<<<(unsigned)grid, threads, 0, st.take()>>>(g, g.counter + slice);
         if (cudaGetLastError() != cudaSuccess) return -1;
         const int r = launch_fock_slices<LA, LB, LC, LD, R, CD0 + S>(g, st, slice + 1);
         return r < 0 ? r : r + 1;

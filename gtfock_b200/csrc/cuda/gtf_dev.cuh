@@ -243,6 +243,16 @@ struct RysArg {
             }
         }
     }
+    // one root, its weight alone ((ss|ss): half the bytes from shared memory)
+    __device__ __forceinline__ R weight() const
+    {
+        constexpr int DEG = RysTab<R>::deg(N);
+        if (row == nullptr) return (R)RYS_LARGE_W[N][0] * b;
+        R w = row[2 * DEG * N + 1];
+#pragma unroll
+        for (int j = DEG - 1; j >= 0; j--) w = gfma(w, a, row[2 * j * N + 1]);
+        return w;
+    }
     __device__ __forceinline__ void root(int r, R &u, R &w) const
     {
         constexpr int DEG = RysTab<R>::deg(N);
@@ -411,7 +421,12 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
             const RysArg<NR, R> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             R u[NR], w[NR];
-            if constexpr (!LOOP) rys.all(u, w);
+            if constexpr (LA + LB + LC + LD == 0) {
+                u[0] = 0;
+                w[0] = rys.weight();
+            } else if constexpr (!LOOP) {
+                rys.all(u, w);
+            }
             const R qf = q_ * ipq, pf = p_ * ipq;
 #pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
@@ -498,7 +513,12 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
             const RysArg<NR, float> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             float u[NR], w[NR];
-            if constexpr (!LOOP) rys.all(u, w);
+            if constexpr (LA + LB + LC + LD == 0) {
+                u[0] = 0;
+                w[0] = rys.weight();
+            } else if constexpr (!LOOP) {
+                rys.all(u, w);
+            }
             const float qf = q * ipq, pf = p * ipq;
 #pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
