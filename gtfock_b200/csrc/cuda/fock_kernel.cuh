@@ -131,42 +131,64 @@ __host__ __device__ constexpr int fock_slice(int LA, int LB, int LC, int LD, int
 
 // One launch per slice (CD0 = first ket component of the slice): each
 // kernel holds the code of a single slice, which keeps the instruction
-// footprint of the d-class kernels small.  The Rys table block of this class
-// (NR roots, precision R) is staged in shared memory by every block.
-// Blocks per SM the register allocation must allow: small quartets run
-// latency-bound dependency chains (Rys polynomial, recurrences), so more
-// resident warps pay off more than the registers they give up.
-__host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD, int slice)
+// footprint of the d-class kernels small.  The class's table (Boys functions
+// for low_class, else the NR-root block of the Rys table; precision R) is
+// staged in shared memory by every block.
+// Blocks (of FOCK_THREADS) per SM the register allocation must allow: small
+// quartets run latency-bound dependency chains (polynomials, recurrences), so
+// more resident warps pay off more than the registers they give up.  C54H18 /
+// cc-pVDZ, FP64 ms with one block fewer, as chosen, one more: (ss|ss) 7.18
+// 6.99 7.11 (of 10), (ps|ss) 21.8 21.2 21.1, (ps|ps) 14.9 15.1 15.5 (but
+// (H2O)64 5.92 5.78 5.97), (ds|ps) 14.6 14.2, (pp|ps) 15.6 13.2 13.9; the Rys
+// classes of 54 integrals lose 25-50% with 3 blocks in FP64 (spills) and gain
+// 3-5% in FP32.  No primitive record is loaded ahead: with this many warps a
+// load's latency is hidden, and the registers of two records more cost
+// 6% of the build in spills.
+__host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD, int fp32)
 {
-    const int nq = ncart(LA) * ncart(LB) * slice;
-    return nq <= 3 ? 6 : nq <= 9 ? 4 : nq <= 27 ? 3 : 2;
+    const int nq = ncart(LA) * ncart(LB) * fock_slice(LA, LB, LC, LD, fp32);
+    if (low_class(LA, LB, LC, LD))
+        return fp32 ? (nq <= 1 ? 10 : nq <= 3 ? 10 : nq <= 9 ? 7 : nq <= 18 ? 5 : 4)
+                    : (nq <= 1 ? 8 : nq <= 3 ? 7 : nq <= 9 ? 5 : nq <= 18 ? 4 : 3);
+    return nq <= (fp32 ? 54 : 36) ? 3 : 2;
 }
 
 //
-// A launch with many units per SM runs one block of fock_max_threads on each,
-// so that the SM holds one copy of the Rys table (13 to 49 KB) and the rest
+// A launch with many units per SM runs one block of fock_max_threads on each
+// (two, of at most 1024 threads), so that the SM holds one copy of the class's
+// table (up to 49 KB) and the rest
 // of its 228 KB caches the gathers of D and of the primitive records; small
 // launches spread blocks of FOCK_THREADS over the SMs.  The registers per
 // thread are the same.
+__host__ __device__ constexpr int fock_big_blocks(int LA, int LB, int LC, int LD, int fp32)
+{
+    return FOCK_THREADS * fock_min_blocks(LA, LB, LC, LD, fp32) > 1024 ? 2 : 1;
+}
 __host__ __device__ constexpr int fock_max_threads(int LA, int LB, int LC, int LD, int fp32)
 {
-    return FOCK_THREADS * fock_min_blocks(LA, LB, LC, LD, fock_slice(LA, LB, LC, LD, fp32));
+    return FOCK_THREADS * fock_min_blocks(LA, LB, LC, LD, fp32) / fock_big_blocks(LA, LB, LC, LD, fp32);
 }
 
 template <int LA, int LB, int LC, int LD, typename R, int CD0, bool BATCH>
-__global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0), 1)
+__global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0),
+                                  fock_big_blocks(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0))
     k_fock(const FockGrid g, unsigned long long *counter)
 {
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NCD = ncart(LC) * ncart(LD);
     constexpr int S = fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
     constexpr int N = (NCD - CD0 < S) ? NCD - CD0 : S;
-    __shared__ __align__(16) R tab[RysTab<R>::len(NR)];
+    constexpr bool LOW = low_class(LA, LB, LC, LD);
+    __shared__ __align__(16) R tab[LOW ? BoysTab<R>::LEN : RysTab<R>::len(NR)];
     // the launch's unit count, kept in shared memory rather than a register
     // across the integral loops (visible after the staging's barrier)
     __shared__ unsigned long long s_nunits;
     if (threadIdx.x == 0) s_nunits = (unsigned long long)(g.nunits_dev ? *g.nunits_dev : g.nunits);
-    rys_stage<R, NR>(tab);
+    if constexpr (LOW) {
+        table_stage<BoysTab<R>::LEN>(tab, BoysTab<R>::ptr(LA + LB + LC));
+    } else {
+        table_stage<RysTab<R>::len(NR)>(tab, RysTab<R>::ptr(NR));
+    }
     const int lane = threadIdx.x & 31;
     // batched launches: per-warp slots for the claimed range of units and the
     // molecule of the current unit, so that neither holds registers across
@@ -263,10 +285,10 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
         for (int k = 0; k < ncart(LA) * ncart(LB) * N; k++) acc[k] = (R)0;
         if constexpr (sizeof(R) == 4) {
             const PPRec32 src{GTF_FLD(pprec32)};
-            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true>(src, pb, pk, acc, tab, split);
+            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true, LOW>(src, pb, pk, acc, tab, split);
         } else {
             const PPRec src{GTF_FLD(pprec)};
-            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true>(src, pb, src, pk, acc, tab, split);
+            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true, LOW>(src, pb, src, pk, acc, tab, split);
         }
         // sum the lanes of each quartet; the first of them digests it
         const int nl = (split & 0xff) * ((split >> 8) & 0xff);
@@ -321,6 +343,7 @@ int launch_fock_slices(const FockGrid &g, FockStreams &st, int slice)
     if constexpr (CD0 < NCD) {
         constexpr int S = fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
         auto k = g.nmol > 1 ? k_fock<LA, LB, LC, LD, R, CD0, true> : k_fock<LA, LB, LC, LD, R, CD0, false>;
+        constexpr int BIG = fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
         // the same on every device this code runs on (sm_100a): asked once
         static std::atomic<int> occ[2];
         int per_sm = occ[g.nmol > 1].load(std::memory_order_relaxed);
@@ -330,13 +353,12 @@ int launch_fock_slices(const FockGrid &g, FockStreams &st, int slice)
             occ[g.nmol > 1].store(per_sm, std::memory_order_relaxed);
         }
         if (g.query) return per_sm;
-        constexpr int BIG = fock_max_threads(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
         int threads = FOCK_THREADS;
         if (g.ctas_per_sm > 0 && g.ctas_per_sm < per_sm) {
             per_sm = g.ctas_per_sm;
         } else if (g.nunits >= (long long)g.nsm * (BIG / 32) * GTF_BIG_ROUNDS) {
             threads = BIG;
-            per_sm = 1;
+            per_sm = fock_big_blocks(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
         }
         long long want = (g.nunits + threads / 32 - 1) / (threads / 32);
         long long grid = (long long)g.nsm * per_sm;

@@ -174,16 +174,16 @@ struct RysTab<float> {
     static __device__ __forceinline__ const float *ptr(int n) { return RYS32_TABLE + off(n); }
 };
 
-// Stages the N-root block into shared memory: 16-byte asynchronous copies,
+// Stages LEN values of a table into shared memory: 16-byte asynchronous copies,
 // all in flight at once.  (A loop of 8-byte loads was one dependent round
 // trip to L2 per thread and pass, up to 46 of them: most of the time of a
 // launch with little work.)
-template <typename R, int N>
-__device__ __forceinline__ void rys_stage(R *stab)
+template <int LEN, typename R>
+__device__ __forceinline__ void table_stage(R *stab, const R *table)
 {
-    constexpr int NV = RysTab<R>::len(N) * (int)sizeof(R) / 16;
-    static_assert(RysTab<R>::len(N) * sizeof(R) % 16 == 0 && RysTab<R>::off(N) * sizeof(R) % 16 == 0, "whole vectors");
-    const char *src = reinterpret_cast<const char *>(RysTab<R>::ptr(N));
+    constexpr int NV = LEN * (int)sizeof(R) / 16;
+    static_assert(LEN * sizeof(R) % 16 == 0, "whole vectors");
+    const char *src = reinterpret_cast<const char *>(table);
     const unsigned dst = (unsigned)__cvta_generic_to_shared(stab);
     for (int k = threadIdx.x; k < NV; k += blockDim.x)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * k), "l"(src + 16 * k) : "memory");
@@ -242,16 +242,6 @@ struct RysArg {
                 w[i] = gfma(w[i], a, t.y);
             }
         }
-    }
-    // one root, its weight alone ((ss|ss): half the bytes from shared memory)
-    __device__ __forceinline__ R weight() const
-    {
-        constexpr int DEG = RysTab<R>::deg(N);
-        if (row == nullptr) return (R)RYS_LARGE_W[N][0] * b;
-        R w = row[2 * DEG * N + 1];
-#pragma unroll
-        for (int j = DEG - 1; j >= 0; j--) w = gfma(w, a, row[2 * j * N + 1]);
-        return w;
     }
     __device__ __forceinline__ void root(int r, R &u, R &w) const
     {
@@ -361,6 +351,8 @@ __device__ __forceinline__ void hrr_abcd(const R (&G)[LA + LB + 1][LC + LD + 1],
     }
 }
 
+#include "eri_low.cuh"
+
 // ---------------------------------------------------------------------------
 // contracted Cartesian (ab|cd), accumulated into acc[ia + NA*(ib + NB*(ic + NC*id))]
 // ---------------------------------------------------------------------------
@@ -378,11 +370,13 @@ __host__ __device__ constexpr int prim_split(int ks, int k0, int bs, int b0)
 // call it once per slice so that a slice's accumulators fit in registers.
 // R = double, or float for quartets evaluated in single precision (the
 // differences of centres are formed in double first, then rounded).
+// LOW: Boys functions and recurrences (eri_low.cuh) instead of Rys quadrature;
+// rtab is then the F_m rows of BOYS_TABLE, m the total angular momentum.
 // rtab: the NR-root block of the Rys table of precision R.
 // Loop order: ket primitive pairs outside (one per lane), bra primitive pairs
 // inside -- the bra is shared by the warp, so its records are warp-uniform
 // loads that stay in L1, and each lane reads its ket's records once.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, class PPB, class PPK,
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool LOW = false, class PPB, class PPK,
           typename R>
 __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec &pb, const PPK &ket,
                                                   const PairRec &pk, R (&acc)[ncart(LA) * ncart(LB) * N],
@@ -391,24 +385,19 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
+    static_assert(!LOW || (low_class(LA, LB, LC, LD) && LD == 0 && N == NC), "whole quartets of the low classes");
+    R low[LOW ? low_nsum(LA, LB, LC) : 1] = {};
     const R ABx = (R)pb.ABx, ABy = (R)pb.ABy, ABz = (R)pb.ABz;
     const R CDx = (R)pk.ABx, CDy = (R)pk.ABy, CDz = (R)pk.ABz;
     const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
-    if (ib0 >= pb.n) return;
-    const PrimVals b0 = bra.get(pb, ib0);
-    PrimVals nk;
-    if (ik0 < pk.n) nk = ket.get(pk, ik0);
+    if (ib0 >= pb.n) return;   // no work: acc stays as it is
     for (int ik = ik0; ik < pk.n; ik += kstep) {
-        const PrimVals kq = nk;
-        if (ik + kstep < pk.n) nk = ket.get(pk, ik + kstep);
-        if (SKIP && fabs(b0.K * kq.K) < GTF_PRIMQ_EPS) break;  // both lists are in descending |K|
+        const PrimVals kq = ket.get(pk, ik);
         const R q_ = (R)kq.p, h2q = (R)kq.h;
         const R QCx = (R)(kq.Px - pk.Ax), QCy = (R)(kq.Py - pk.Ay), QCz = (R)(kq.Pz - pk.Az);
-        // the next bra primitive pair is loaded while the current one is used
-        PrimVals nb = b0;
-        for (int ib = ib0; ib < pb.n; ib += bstep) {
-            const PrimVals bq = nb;
-            if (ib + bstep < pb.n) nb = bra.get(pb, ib + bstep);
+        int ib = ib0;
+        for (; ib < pb.n; ib += bstep) {
+            const PrimVals bq = bra.get(pb, ib);
             if (SKIP && fabs(bq.K * kq.K) < GTF_PRIMQ_EPS) break;
             const R p_ = (R)bq.p, h2p = (R)bq.h;
             const R PAx = (R)(bq.Px - pb.Ax), PAy = (R)(bq.Py - pb.Ay), PAz = (R)(bq.Pz - pb.Az);
@@ -418,15 +407,20 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
             const R rho = p_ * q_ * ipq;
             const R T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
             const R pref = (R)(bq.K * kq.K) * rpq;
+            if constexpr (LOW) {
+                const R qf = q_ * ipq, pf = p_ * ipq;
+                R S[LA + LB + LC + 1];
+                boys<LA + LB + LC>(T, S, rtab);
+#pragma unroll
+                for (int m = 0; m <= LA + LB + LC; m++) S[m] *= pref;
+                const R PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
+                low_prim<LA, LB, LC>(low, S, PA, QC, PQ, qf, pf, h2p, (R)0.5 * ipq);
+                continue;
+            }
             const RysArg<NR, R> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             R u[NR], w[NR];
-            if constexpr (LA + LB + LC + LD == 0) {
-                u[0] = 0;
-                w[0] = rys.weight();
-            } else if constexpr (!LOOP) {
-                rys.all(u, w);
-            }
+            if constexpr (!LOOP) rys.all(u, w);
             const R qf = q_ * ipq, pf = p_ * ipq;
 #pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
@@ -467,6 +461,12 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
                 }
             }
         }
+        // not one bra primitive: both lists are in descending |K|
+        if (SKIP && ib == ib0) break;
+    }
+    if constexpr (LOW) {
+        const R AB[3] = {ABx, ABy, ABz};
+        low_finish<LA, LB, LC>(low, AB, acc);
     }
     (void)ND;
 }
@@ -474,7 +474,7 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
 // FP32 quartets: everything in single precision, from the FP32 records (centres
 // relative to each pair's first shell; P - Q = PA - QC + (A - C) with A - C
 // formed in double once per quartet).  Same structure as eri_accumulate_cd.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP>
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool LOW = false>
 __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const PairRec &pb, const PairRec &pk,
                                                     float (&acc)[ncart(LA) * ncart(LB) * N], const float *rtab,
                                                     int split = prim_split(1, 0, 1, 0))
@@ -482,25 +482,20 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC);
+    float low[LOW ? low_nsum(LA, LB, LC) : 1] = {};
     const float ABx = (float)pb.ABx, ABy = (float)pb.ABy, ABz = (float)pb.ABz;
     const float CDx = (float)pk.ABx, CDy = (float)pk.ABy, CDz = (float)pk.ABz;
     const float ACx = (float)(pb.Ax - pk.Ax), ACy = (float)(pb.Ay - pk.Ay), ACz = (float)(pb.Az - pk.Az);
     const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
-    if (ib0 >= pb.n) return;
-    const PrimVals32 b0 = src.get(pb, ib0);
-    PrimVals32 nk;
-    if (ik0 < pk.n) nk = src.get(pk, ik0);
+    if (ib0 >= pb.n) return;   // no work: acc stays as it is
     for (int ik = ik0; ik < pk.n; ik += kstep) {
-        const PrimVals32 kq = nk;
-        if (ik + kstep < pk.n) nk = src.get(pk, ik + kstep);
-        if (SKIP && fabsf(b0.K * kq.K) < (float)GTF_PRIMQ_EPS) break;
+        const PrimVals32 kq = src.get(pk, ik);
         const float q = kq.p, h2q = kq.h;
         const float QCx = kq.PAx, QCy = kq.PAy, QCz = kq.PAz;
         const float dx = ACx - QCx, dy = ACy - QCy, dz = ACz - QCz;
-        PrimVals32 nb = b0;
-        for (int ib = ib0; ib < pb.n; ib += bstep) {
-            const PrimVals32 bq = nb;
-            if (ib + bstep < pb.n) nb = src.get(pb, ib + bstep);
+        int ib = ib0;
+        for (; ib < pb.n; ib += bstep) {
+            const PrimVals32 bq = src.get(pb, ib);
             if (SKIP && fabsf(bq.K * kq.K) < (float)GTF_PRIMQ_EPS) break;
             const float p = bq.p, h2p = bq.h;
             const float PAx = bq.PAx, PAy = bq.PAy, PAz = bq.PAz;
@@ -510,15 +505,20 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
             const float rho = p * q * ipq;
             const float T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
             const float pref = bq.K * kq.K * rpq;
+            if constexpr (LOW) {
+                const float qf = q * ipq, pf = p * ipq;
+                float S[LA + LB + LC + 1];
+                boys<LA + LB + LC>(T, S, rtab);
+#pragma unroll
+                for (int m = 0; m <= LA + LB + LC; m++) S[m] *= pref;
+                const float PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
+                low_prim<LA, LB, LC>(low, S, PA, QC, PQ, qf, pf, h2p, (float)0.5 * ipq);
+                continue;
+            }
             const RysArg<NR, float> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             float u[NR], w[NR];
-            if constexpr (LA + LB + LC + LD == 0) {
-                u[0] = 0;
-                w[0] = rys.weight();
-            } else if constexpr (!LOOP) {
-                rys.all(u, w);
-            }
+            if constexpr (!LOOP) rys.all(u, w);
             const float qf = q * ipq, pf = p * ipq;
 #pragma unroll(LOOP ? 1 : NR)
             for (int r = 0; r < NR; r++) {
@@ -558,6 +558,12 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
                 }
             }
         }
+        // not one bra primitive: both lists are in descending |K|
+        if (SKIP && ib == ib0) break;
+    }
+    if constexpr (LOW) {
+        const float AB[3] = {ABx, ABy, ABz};
+        low_finish<LA, LB, LC>(low, AB, acc);
     }
 }
 

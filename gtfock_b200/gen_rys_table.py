@@ -19,6 +19,11 @@ Method (published, restated here):
   * for T >= TMAX[n] the large-T form is exact to double precision:
     u_i = x_i^2 / T, w_i = W_i / sqrt(T) with x_i > 0 the roots of the Hermite
     polynomial H_2n and W_i their Gauss-Hermite weights.
+The classes of total angular momentum up to 3 need only Boys functions
+F_0 .. F_m: per m and interval of width HB a polynomial for F_m and exp(-T) at
+the middle; exp(-T) elsewhere in the interval is that times a polynomial for
+exp(-s), and F_m-1 .. F_0 follow by the downward recursion
+F_k-1 = (2 T F_k + exp(-T)) / (2k - 1).
 Accuracy of the double table against the 60-digit values: <= 1e-15 relative
 (checked by tests/test_oracle.py against values recomputed here).
 
@@ -41,6 +46,12 @@ TMAX = {1: 40.0, 2: 48.0, 3: 56.0, 4: 62.0, 5: 70.0}
 # single-precision table for the mixed-precision kernels
 H32 = 2.0
 DEG32 = 7
+# Boys functions: interval width, range, degrees of F_m and of exp(-s)
+HB = 0.5
+TB = 48.0
+BMAX = 3
+DEGB = {64: 9, 32: 5}
+DEGE = {64: 10, 32: 5}
 DPS = 60
 
 
@@ -109,6 +120,24 @@ def fit_interval(args):
         return coefs   # [func][coef]
 
 
+def chebyshev_fit(f, h, deg):
+    """Monomial coefficients on |s| <= h / 2 of the interpolant of f(s) at the Chebyshev points."""
+    with mp.workdps(DPS):
+        xs = [mp.cos(mp.pi * (2 * k + 1) / (2 * (deg + 1))) for k in range(deg + 1)]
+        V = mp.matrix([[(h * x / 2) ** j for j in range(deg + 1)] for x in xs])
+        c = mp.lu_solve(V, mp.matrix([f(h * x / 2) for x in xs]))
+        return [c[j] for j in range(deg + 1)]
+
+
+def fit_boys(args):
+    m, k, deg = args
+    with mp.workdps(DPS):
+        mid = mp.mpf((k + 0.5) * HB)
+        return chebyshev_fit(lambda s: boys_moments(mid + s, 2)[0] if m == 0 else
+                             mp.hyp1f1(m + mp.mpf(1) / 2, m + mp.mpf(3) / 2, -(mid + s)) / (2 * m + 1),
+                             HB, deg) + [mp.exp(-mid)]
+
+
 def build_table(h, deg, pool):
     """h, deg: per root count (dict) or one value for all"""
     tables = {}
@@ -149,6 +178,9 @@ def main(out_path=None):
     with mproc.get_context("spawn").Pool(os.cpu_count()) as pool:
         t64 = build_table(H64, DEG64, pool)
         t32 = build_table(H32, DEG32, pool)
+        nb = int(round(TB / HB))
+        boys = {p: [pool.map(fit_boys, [(m, k, DEGB[p]) for k in range(nb)]) for m in range(BMAX + 1)]
+                for p in (64, 32)}
     lines = []
     w = lines.append
     w("/* rys_table.h -- generated by gtfock_b200/gen_rys_table.py; do not edit.")
@@ -212,6 +244,21 @@ def main(out_path=None):
     for n in range(1, NMAX + 1):
         w("  {" + ", ".join(fmt(wt) for _, wt in hl[n]) + "},")
     w("};")
+    # Boys functions: [m][interval][coefficients of F_m, exp(-T_mid)]
+    w("#define BOYS_MMAX %d" % BMAX)
+    w("#define BOYS_H %.1f" % HB)
+    w("#define BOYS_TMAX %.1f" % TB)
+    w("#define BOYS_NINT %d" % nb)
+    for p, name, typ in ((64, "BOYS", "double"), (32, "BOYS32", "float")):
+        w("#define %s_DEG %d" % (name, DEGB[p]))
+        w("#define %s_EXP_DEG %d" % (name, DEGE[p]))
+        w("#define %s_EXP_LIST %s" % (name, ", ".join(
+            fmt(c, p == 32) for c in chebyshev_fit(lambda s: mp.exp(-s), mp.mpf(HB), DEGE[p]))))
+        vals = [c for m in range(BMAX + 1) for row in boys[p][m] for c in row]
+        w("RYS_QUAL const %s %s_TABLE[%d] = {" % (typ, name, len(vals)))
+        for i in range(0, len(vals), 4):
+            w("  " + ", ".join(fmt(x, p == 32) for x in vals[i:i + 4]) + ",")
+        w("};")
     with open(out_path, "w") as f:
         f.write("\n".join(lines) + "\n")
     print("wrote", out_path, len(flat), "doubles,", len(flat32), "floats")
