@@ -148,8 +148,8 @@ __host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD
 {
     const int nq = ncart(LA) * ncart(LB) * fock_slice(LA, LB, LC, LD, fp32);
     if (low_class(LA, LB, LC, LD))
-        return fp32 ? (nq <= 1 ? 10 : nq <= 3 ? 10 : nq <= 9 ? 7 : nq <= 18 ? 5 : 4)
-                    : (nq <= 1 ? 8 : nq <= 3 ? 7 : nq <= 9 ? 5 : nq <= 18 ? 4 : 3);
+        return fp32 ? (nq <= 1 ? 10 : nq <= 3 ? 10 : nq <= 9 ? 7 : nq <= 18 ? 5 : nq <= 27 ? 4 : 3)
+                    : (nq <= 1 ? 8 : nq <= 3 ? 7 : nq <= 9 ? 5 : nq <= 18 ? 4 : nq <= 27 ? 3 : 2);
     return nq <= (fp32 ? 54 : 36) ? 3 : 2;
 }
 
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
     __shared__ unsigned long long s_nunits;
     if (threadIdx.x == 0) s_nunits = (unsigned long long)(g.nunits_dev ? *g.nunits_dev : g.nunits);
     if constexpr (LOW) {
-        table_stage<BoysTab<R>::LEN>(tab, BoysTab<R>::ptr(LA + LB + LC));
+        table_stage<BoysTab<R>::LEN>(tab, BoysTab<R>::ptr(LA + LB + LC + LD));
     } else {
         table_stage<RysTab<R>::len(NR)>(tab, RysTab<R>::ptr(NR));
     }

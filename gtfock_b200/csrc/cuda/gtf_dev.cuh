@@ -385,8 +385,8 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
-    static_assert(!LOW || (low_class(LA, LB, LC, LD) && LD == 0 && N == NC), "whole quartets of the low classes");
-    R low[LOW ? low_nsum(LA, LB, LC) : 1] = {};
+    static_assert(!LOW || (low_class(LA, LB, LC, LD) && N == NC * ND), "whole quartets of the low classes");
+    R low[LOW ? low_nsum(LA, LB, LC, LD) : 1] = {};
     const R ABx = (R)pb.ABx, ABy = (R)pb.ABy, ABz = (R)pb.ABz;
     const R CDx = (R)pk.ABx, CDy = (R)pk.ABy, CDz = (R)pk.ABz;
     const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
@@ -409,12 +409,12 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
             const R pref = (R)(bq.K * kq.K) * rpq;
             if constexpr (LOW) {
                 const R qf = q_ * ipq, pf = p_ * ipq;
-                R S[LA + LB + LC + 1];
-                boys<LA + LB + LC>(T, S, rtab);
+                R S[LA + LB + LC + LD + 1];
+                boys<LA + LB + LC + LD>(T, S, rtab);
 #pragma unroll
-                for (int m = 0; m <= LA + LB + LC; m++) S[m] *= pref;
+                for (int m = 0; m <= LA + LB + LC + LD; m++) S[m] *= pref;
                 const R PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
-                low_prim<LA, LB, LC>(low, S, PA, QC, PQ, qf, pf, h2p, (R)0.5 * ipq);
+                low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (R)0.5 * ipq);
                 continue;
             }
             const RysArg<NR, R> rys(T, rtab);
@@ -465,8 +465,8 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
         if (SKIP && ib == ib0) break;
     }
     if constexpr (LOW) {
-        const R AB[3] = {ABx, ABy, ABz};
-        low_finish<LA, LB, LC>(low, AB, acc);
+        const R AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
+        low_finish<LA, LB, LC, LD>(low, AB, CD, acc);
     }
     (void)ND;
 }
@@ -482,7 +482,7 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC);
-    float low[LOW ? low_nsum(LA, LB, LC) : 1] = {};
+    float low[LOW ? low_nsum(LA, LB, LC, LD) : 1] = {};
     const float ABx = (float)pb.ABx, ABy = (float)pb.ABy, ABz = (float)pb.ABz;
     const float CDx = (float)pk.ABx, CDy = (float)pk.ABy, CDz = (float)pk.ABz;
     const float ACx = (float)(pb.Ax - pk.Ax), ACy = (float)(pb.Ay - pk.Ay), ACz = (float)(pb.Az - pk.Az);
@@ -507,12 +507,12 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
             const float pref = bq.K * kq.K * rpq;
             if constexpr (LOW) {
                 const float qf = q * ipq, pf = p * ipq;
-                float S[LA + LB + LC + 1];
-                boys<LA + LB + LC>(T, S, rtab);
+                float S[LA + LB + LC + LD + 1];
+                boys<LA + LB + LC + LD>(T, S, rtab);
 #pragma unroll
-                for (int m = 0; m <= LA + LB + LC; m++) S[m] *= pref;
+                for (int m = 0; m <= LA + LB + LC + LD; m++) S[m] *= pref;
                 const float PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
-                low_prim<LA, LB, LC>(low, S, PA, QC, PQ, qf, pf, h2p, (float)0.5 * ipq);
+                low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (float)0.5 * ipq);
                 continue;
             }
             const RysArg<NR, float> rys(T, rtab);
@@ -562,8 +562,8 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
         if (SKIP && ib == ib0) break;
     }
     if constexpr (LOW) {
-        const float AB[3] = {ABx, ABy, ABz};
-        low_finish<LA, LB, LC>(low, AB, acc);
+        const float AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
+        low_finish<LA, LB, LC, LD>(low, AB, CD, acc);
     }
 }
 

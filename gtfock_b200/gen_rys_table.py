@@ -19,7 +19,7 @@ Method (published, restated here):
   * for T >= TMAX[n] the large-T form is exact to double precision:
     u_i = x_i^2 / T, w_i = W_i / sqrt(T) with x_i > 0 the roots of the Hermite
     polynomial H_2n and W_i their Gauss-Hermite weights.
-The classes of total angular momentum up to 3 need only Boys functions
+The light classes (total angular momentum up to 4) need only Boys functions
 F_0 .. F_m: per m and interval of width HB a polynomial for F_m and exp(-T) at
 the middle; exp(-T) elsewhere in the interval is that times a polynomial for
 exp(-s), and F_m-1 .. F_0 follow by the downward recursion
@@ -49,7 +49,7 @@ DEG32 = 7
 # Boys functions: interval width, range, degrees of F_m and of exp(-s)
 HB = 0.5
 TB = 48.0
-BMAX = 3
+BMAX = 4
 DEGB = {64: 9, 32: 5}
 DEGE = {64: 10, 32: 5}
 DPS = 60
