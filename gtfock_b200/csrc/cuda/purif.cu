@@ -71,7 +71,7 @@ static size_t part_len(int n)
     return a > b ? a : b;
 }
 
-// row-major C = A B^T (pdgemm3D_2) and C = A B, via column-major cuBLAS
+// row-major C = A B^T (pdgemm3D_2), via column-major cuBLAS
 static int gemm_abt(gtf_purif_dev *p, const double *A, const double *B, double *C)
 {
     const double one = 1.0, zero = 0.0;
@@ -79,10 +79,112 @@ static int gemm_abt(gtf_purif_dev *p, const double *A, const double *B, double *
     return GTF_OK;
 }
 
-static int gemm_ab(gtf_purif_dev *p, const double *A, const double *B, double *C)
+// ---------------------------------------------------------------------------
+// C = A B^T for products that are symmetric (D D and D D^2 of a symmetric D):
+// the tiles on and below the diagonal, mirrored.  Row-major n x n.
+//
+// One block per 32 x 32 tile; its four warps share the K loop (each takes 8 of
+// a slab's 32) and hold the whole tile in FP64 tensor-core accumulators
+// (m8n8k4: 16 products per 8 fragment loads), summed through shared memory at
+// the end.  Bound by the FP64 pipe; at 846 functions the 378 tiles are one
+// wave of three blocks per SM.  cuBLAS's full product in 729 such tiles took
+// 57 us there.
+// ---------------------------------------------------------------------------
+#define ST_TILE 32
+#define ST_LD 36   // row stride in doubles: the 4 x 4 elements a half warp reads are in different banks
+
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool ok)
 {
-    const double one = 1.0, zero = 0.0;
-    CKB(cublasDgemm(p->blas, CUBLAS_OP_N, CUBLAS_OP_N, p->n, p->n, p->n, &one, B, p->n, A, p->n, &zero, C, p->n));
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
+}
+
+__global__ void __launch_bounds__(128) k_sym_abt(const double *__restrict__ A, const double *__restrict__ B,
+                                                 double *__restrict__ C, int n)
+{
+    __shared__ __align__(16) double buf[2][2][ST_TILE * ST_LD];   // [stage][A or B]
+    // tile (ti, tj), tj <= ti, of the linear index ti (ti + 1) / 2 + tj
+    int ti = (int)((sqrtf(8.0f * (float)blockIdx.x + 1.0f) - 1.0f) * 0.5f);
+    while (ti * (ti + 1) / 2 > (int)blockIdx.x) ti--;
+    while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ti++;
+    const int tj = (int)blockIdx.x - ti * (ti + 1) / 2;
+    const int r0 = ti * ST_TILE, c0 = tj * ST_TILE;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto load = [&](int stage, int k0) {
+#pragma unroll
+        for (int q = 0; q < ST_TILE * ST_TILE / 128; q++) {
+            const int e = threadIdx.x + 128 * q, r = e / ST_TILE, k = e % ST_TILE;
+            const bool ka = k0 + k < n, oa = ka && r0 + r < n, ob = ka && c0 + r < n;
+            cp_async8(&buf[stage][0][r * ST_LD + k], oa ? A + (size_t)(r0 + r) * n + k0 + k : A, oa);
+            cp_async8(&buf[stage][1][r * ST_LD + k], ob ? B + (size_t)(c0 + r) * n + k0 + k : B, ob);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    double acc[4][4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    load(0, 0);
+    int st = 0;
+    for (int k0 = 0; k0 < n; k0 += ST_TILE, st ^= 1) {
+        if (k0 + ST_TILE < n) {
+            load(st ^ 1, k0 + ST_TILE);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        // fragments: A row lane / 4, k lane % 4; B column lane / 4, k lane % 4
+        const int o = (lane >> 2) * ST_LD + 8 * w + (lane & 3);
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) {
+            double a[4], b[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                a[i] = buf[st][0][o + 8 * i * ST_LD + k];
+                b[i] = buf[st][1][o + 8 * i * ST_LD + k];
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++)
+                    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                                 : "+d"(acc[i][j][0]), "+d"(acc[i][j][1])
+                                 : "d"(a[i]), "d"(b[j]));
+        }
+        __syncthreads();
+    }
+    // the four warps' sums: 32 x 32 each, row stride 33
+    double *part = &buf[0][0][0];
+    static_assert(4 * ST_TILE * 33 <= 4 * ST_TILE * ST_LD, "partial tiles fit the stages");
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int q = 0; q < 2; q++)
+                part[w * ST_TILE * 33 + (8 * i + (lane >> 2)) * 33 + 8 * j + 2 * (lane & 3) + q] = acc[i][j][q];
+    __syncthreads();
+    for (int e = threadIdx.x; e < ST_TILE * ST_TILE; e += 128) {
+        const int r = e / ST_TILE, c = e % ST_TILE;
+        double *p = part + r * 33 + c;
+        p[0] = (p[0] + p[ST_TILE * 33]) + (p[2 * ST_TILE * 33] + p[3 * ST_TILE * 33]);
+        if (r0 + r < n && c0 + c <= r0 + r) C[(size_t)(r0 + r) * n + c0 + c] = p[0];
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < ST_TILE * ST_TILE; e += 128) {
+        const int c = e / ST_TILE, r = e % ST_TILE;
+        if (r0 + r < n && c0 + c < r0 + r) C[(size_t)(c0 + c) * n + r0 + r] = part[r * 33 + c];
+    }
+}
+
+static int sym_abt(gtf_purif_dev *p, const double *A, const double *B, double *C)
+{
+    const int nt = (p->n + ST_TILE - 1) / ST_TILE;
+    k_sym_abt<<<nt * (nt + 1) / 2, 128, 0, p->st>>>(A, B, C, p->n);
+    CKP(cudaGetLastError());
+    gtf_note_launches(1);
     return GTF_OK;
 }
 
@@ -512,8 +614,8 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
     bool stopped = false;
     for (it = 0; it < PUR_MAX_ITERS && !stopped;) {
         for (int k = 0; k < PURIF_CHECK && it < PUR_MAX_ITERS; k++, it++) {
-            if (gemm_abt(p, p->D, p->D, p->D2)) return GTF_ERR_CUDA;
-            if (gemm_ab(p, p->D, p->D2, p->D3)) return GTF_ERR_CUDA;
+            if (sym_abt(p, p->D, p->D, p->D2)) return GTF_ERR_CUDA;
+            if (sym_abt(p, p->D, p->D2, p->D3)) return GTF_ERR_CUDA;
             k_purif_stats<<<RED_BLOCKS, RED_THREADS, 0, st>>>(p->D, p->D2, p->D3, n, p->part);
             k_purif_finish<<<1, 32, 0, st>>>(p->part, RED_BLOCKS, p->scal);
             k_purif_update<<<ge, 256, 0, st>>>(p->D, p->D2, p->D3, nn, p->scal);
