@@ -427,6 +427,129 @@ __global__ void __launch_bounds__(BJ_THREADS) k_j_pur_step(const JobDev *__restr
     }
 }
 
+// Jobs of at most BJ_SMALL functions: the whole purification in one launch,
+// one block per job, P, P^2 and P^3 in shared memory (223 KB at 96
+// functions).  A step of a few small jobs took two product launches and a
+// step launch, 29 us whatever the size, and a host wait every BJ_PUR_CHECK of
+// them; here it takes 3 us at 30 functions and 15 us at 69.  The products and
+// sums add in the order of k_bgemm and k_j_pur_step, so the numbers are the same.
+#define BJ_SMALL 96
+
+// C = A B^T (TB) or A B over the block: thread (ti, tj) of 16 x 16 has rows
+// ti + 16 r and columns tj + 16 c, r, c < NB, of matrices with an odd row
+// stride (a warp's 16 rows of B^T are then in different banks)
+template <int NB, bool TB>
+__device__ __forceinline__ void small_gemm(const double *A, const double *B, double *C, int n, int ld)
+{
+    const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+    double acc[NB][NB];
+#pragma unroll
+    for (int r = 0; r < NB; r++)
+#pragma unroll
+        for (int c = 0; c < NB; c++) acc[r][c] = 0.0;
+    // rows and columns beyond the matrix read the last one and are not stored
+    int ra[NB], cb[NB];
+#pragma unroll
+    for (int q = 0; q < NB; q++) {
+        ra[q] = min(ti + 16 * q, n - 1) * ld;
+        cb[q] = TB ? min(tj + 16 * q, n - 1) * ld : min(tj + 16 * q, n - 1);
+    }
+    for (int k = 0; k < n; k++) {
+        double a[NB], b[NB];
+#pragma unroll
+        for (int q = 0; q < NB; q++) {
+            a[q] = A[ra[q] + k];
+            b[q] = TB ? B[cb[q] + k] : B[k * ld + cb[q]];
+        }
+#pragma unroll
+        for (int r = 0; r < NB; r++)
+#pragma unroll
+            for (int c = 0; c < NB; c++) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+    }
+#pragma unroll
+    for (int r = 0; r < NB; r++)
+#pragma unroll
+        for (int c = 0; c < NB; c++) {
+            const int i = ti + 16 * r, j = tj + 16 * c;
+            if (i < n && j < n) C[i * ld + j] = acc[r][c];
+        }
+}
+
+template <bool TB>
+__device__ __forceinline__ void small_gemm_any(const double *A, const double *B, double *C, int n, int ld)
+{
+    switch ((n + 15) / 16) {
+        case 1: small_gemm<1, TB>(A, B, C, n, ld); break;
+        case 2: small_gemm<2, TB>(A, B, C, n, ld); break;
+        case 3: small_gemm<3, TB>(A, B, C, n, ld); break;
+        case 4: small_gemm<4, TB>(A, B, C, n, ld); break;
+        case 5: small_gemm<5, TB>(A, B, C, n, ld); break;
+        default: small_gemm<6, TB>(A, B, C, n, ld); break;
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(BJ_THREADS) k_j_pur_small(const JobDev *__restrict__ jobs, const int *__restrict__ list,
+                                                           double *__restrict__ scal, int *__restrict__ active,
+                                                           int *__restrict__ iters)
+{
+    static_assert(BJ_THREADS == 256 && BJ_SMALL <= 96, "16 x 16 threads, up to 6 x 6 elements each");
+    extern __shared__ double small_mem[];
+    __shared__ double sh[BJ_THREADS];
+    const int q = list[blockIdx.x];
+    const JobDev j = jobs[q];
+    const int n = j.n, ld = n | 1, nn = n * n;
+    double *P = small_mem, *P2 = P + n * ld, *P3 = P2 + n * ld;
+    for (int k = threadIdx.x; k < nn; k += BJ_THREADS) P[(k / n) * ld + k % n] = j.P[k];
+    __syncthreads();
+    double best = 0.0, stall = 0.0, err = 0.0;   // the same in every thread
+    int it = 0;
+    bool run = true;
+    while (run && it < BJ_PUR_MAX) {
+        small_gemm_any<true>(P, P, P2, n, ld);
+        small_gemm_any<false>(P, P2, P3, n, ld);
+        double e = 0.0, t = 0.0, t2 = 0.0;
+        for (int k = threadIdx.x; k < nn; k += BJ_THREADS) {
+            const int o = (k / n) * ld + k % n;
+            const double d = P[o] - P2[o];
+            e += d * d;
+        }
+        for (int i = threadIdx.x; i < n; i += BJ_THREADS) {
+            const int o = i * ld + i;
+            t += P2[o] - P3[o];
+            t2 += P[o] - P2[o];
+        }
+        e = block_sum(e, sh);
+        t = block_sum(t, sh);
+        t2 = block_sum(t2, sh);
+        const double c = t / t2;
+        const bool ok = isfinite(c) && c >= -0.25 && c <= 1.25;   // as k_j_pur_step
+        err = ok ? sqrt(e) : 0.0;
+        for (int k = threadIdx.x; k < nn && ok; k += BJ_THREADS) {
+            const int o = (k / n) * ld + k % n;
+            if (c < 0.5) P[o] = ((1.0 - 2.0 * c) * P[o] + (1.0 + c) * P2[o] - P3[o]) / (1.0 - c);
+            else P[o] = ((1.0 + c) * P2[o] - P3[o]) / c;
+        }
+        it++;
+        if (ok) {
+            if (best == 0.0 || err < 0.99 * best) {
+                best = err;
+                stall = 0.0;
+            } else {
+                stall += 1.0;
+            }
+        }
+        run = !(err < 1e-11 || (best < 1e-8 && stall >= 8.0));
+        __syncthreads();
+    }
+    for (int k = threadIdx.x; k < nn; k += BJ_THREADS) j.P[k] = P[(k / n) * ld + k % n];
+    if (threadIdx.x == 0) {
+        scal[q * 8 + 2] = err;
+        iters[q] = it;
+        active[q] = run ? 1 : 0;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -870,8 +993,15 @@ static int rebuild_fock_batch(gtf_batch *b, const std::vector<int> &run)
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
     }
-    // tile shape of the dense products: tuned for this size, else the default
-    b->gshape = 0;
+    // tile shape of the dense products: tuned for this size, else 64 x 64, or
+    // 32 x 32 where those tiles would leave SMs idle
+    long long tiles = 0;
+    for (int s : run)
+        if (!b->jobs[s].pd) tiles += (long long)((b->jobs[s].n + 63) / 64) * ((b->jobs[s].n + 63) / 64);
+    int dev = 0, nsm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    b->gshape = tiles < nsm ? 1 : 0;
     int shape = 0;
     if (gtf_tune_get(2, -1, -1, 0, batch_gemm_work(b, run), &shape, nullptr) && shape >= 0 && shape < BG_NSHAPES)
         b->gshape = shape;
@@ -885,7 +1015,7 @@ extern "C" int gtf_batch_step(gtf_batch_t *b)
     for (int s = 0; s < b->capacity; s++)
         if (b->jobs[s].used && !b->jobs[s].done) run.push_back(s);
     if (run.empty()) return 0;
-    int launches = 0;
+    int launches = 0, pur_steps = 0;
     // ---- Fock build of every running job ----
     if (b->dirty || run != b->fb_members) {
         const int r = rebuild_fock_batch(b, run);
@@ -1014,18 +1144,44 @@ extern "C" int gtf_batch_step(gtf_batch_t *b)
         k_j_pur_init<<<C, BJ_THREADS, 0, b->st>>>(b->d_jobs, b->d_scal, b->d_active);
         CKH(cudaGetLastError());
         launches++;
+        // small jobs purify in one launch; the list of the others follows theirs
+        int nsmall = 0, nact = 0, msmall = 0;
+        for (int q = 0; q < C; q++)
+            if (b->h_jobs[q].n <= BJ_SMALL) {
+                b->h_list[nsmall++] = q;
+                msmall = b->h_jobs[q].n > msmall ? b->h_jobs[q].n : msmall;
+            }
+        for (int q = 0; q < C; q++)
+            if (b->h_jobs[q].n > BJ_SMALL) {
+                const JobDev &d = b->h_jobs[q];
+                set_gemm(b, 6, nact, d.P, d.P, d.P2, d.n, q);
+                set_gemm(b, 7, nact, d.P, d.P2, d.P3, d.n, q);
+                b->h_list[nsmall + nact++] = q;
+            }
+        CKH(cudaMemcpyAsync(b->d_list, b->h_list, sizeof(int) * C, cudaMemcpyHostToDevice, b->st));
+        if (nsmall > 0) {
+            const int smem = 3 * (int)sizeof(double) * msmall * (msmall | 1);
+            // the same value for every batch: lanes on other threads launch too
+            CKH(cudaFuncSetAttribute((const void *)k_j_pur_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     3 * (int)sizeof(double) * BJ_SMALL * (BJ_SMALL | 1)));
+            k_j_pur_small<<<nsmall, BJ_THREADS, smem, b->st>>>(b->d_jobs, b->d_list, b->d_scal, b->d_active, b->d_iters);
+            CKH(cudaGetLastError());
+            launches++;
+        }
         // the launches cover the jobs still purifying: every BJ_PUR_CHECK steps
         // the active flags come back and the job list and the descriptors of
         // the two products are compacted to the jobs that remain
-        int nact = C;
-        for (int q = 0; q < C; q++) b->h_list[q] = q;
-        CKH(cudaMemcpyAsync(b->d_list, b->h_list, sizeof(int) * C, cudaMemcpyHostToDevice, b->st));
+        if (nsmall > 0 && nact > 0) {
+            CKH(cudaMemcpyAsync(b->d_gd + 6 * (size_t)b->capacity, b->h_gd + 6 * (size_t)b->capacity,
+                                sizeof(GemmDesc) * 2 * b->capacity, cudaMemcpyHostToDevice, b->st));
+            CKH(cudaMemcpyAsync(b->d_tp + 6 * C1, b->h_tp + 6 * C1, sizeof(int) * 2 * C1, cudaMemcpyHostToDevice, b->st));
+        }
         int step;
-        for (step = 0; step < BJ_PUR_MAX; step++) {
+        for (step = 0; step < BJ_PUR_MAX && nact > 0; step++) {
             if (run_gemm(b, 6, nact, true, b->d_active, &launches) ||
                 run_gemm(b, 7, nact, false, b->d_active, &launches))
                 return -4;
-            k_j_pur_step<<<nact, BJ_THREADS, 0, b->st>>>(b->d_jobs, b->d_list, b->d_scal, b->d_active, b->d_iters);
+            k_j_pur_step<<<nact, BJ_THREADS, 0, b->st>>>(b->d_jobs, b->d_list + nsmall, b->d_scal, b->d_active, b->d_iters);
             CKH(cudaGetLastError());
             launches++;
             if ((step + 1) % BJ_PUR_CHECK == 0) {
@@ -1033,11 +1189,11 @@ extern "C" int gtf_batch_step(gtf_batch_t *b)
                 CKH(cudaStreamSynchronize(b->st));
                 int m = 0;
                 for (int q = 0; q < C; q++)
-                    if (b->h_act[q]) {
+                    if (b->h_act[q] && b->h_jobs[q].n > BJ_SMALL) {
                         const JobDev &d = b->h_jobs[q];
                         set_gemm(b, 6, m, d.P, d.P, d.P2, d.n, q);
                         set_gemm(b, 7, m, d.P, d.P2, d.P3, d.n, q);
-                        b->h_list[m++] = q;
+                        b->h_list[nsmall + m++] = q;
                     }
                 if (m == 0) break;
                 if (m < nact) {
@@ -1047,11 +1203,11 @@ extern "C" int gtf_batch_step(gtf_batch_t *b)
                                         sizeof(GemmDesc) * 2 * b->capacity, cudaMemcpyHostToDevice, b->st));
                     CKH(cudaMemcpyAsync(b->d_tp + 6 * C1, b->h_tp + 6 * C1, sizeof(int) * 2 * C1,
                                         cudaMemcpyHostToDevice, b->st));
-                    CKH(cudaMemcpyAsync(b->d_list, b->h_list, sizeof(int) * nact, cudaMemcpyHostToDevice, b->st));
+                    CKH(cudaMemcpyAsync(b->d_list + nsmall, b->h_list + nsmall, sizeof(int) * nact, cudaMemcpyHostToDevice, b->st));
                 }
             }
         }
-        b->pur_steps += step + 1;
+        pur_steps = step > 0 ? step + 1 : 0;
         // D_AO = X P X^T (pscf/purif.c:469-476), into the engine's density
         if (run_gemm(b, 8, C, true, nullptr, &launches) || run_gemm(b, 9, C, true, nullptr, &launches)) return -4;
         CKH(cudaMemcpyAsync(b->h_iters, b->d_iters, sizeof(int) * C, cudaMemcpyDeviceToHost, b->st));
@@ -1074,7 +1230,9 @@ extern "C" int gtf_batch_step(gtf_batch_t *b)
         BJob &j = b->jobs[run[cont[q]]];
         j.pur_iters = b->h_iters[q];
         j.pur_total += j.pur_iters;
+        if (j.n <= BJ_SMALL && j.pur_iters > pur_steps) pur_steps = j.pur_iters;
     }
+    b->pur_steps += pur_steps;
     float ms1 = 0.0f, ms2 = 0.0f, ms3 = 0.0f, ms4 = 0.0f;
     cudaEventElapsedTime(&ms1, b->e0, b->e1);
     cudaEventElapsedTime(&ms2, b->e1, b->e2);
