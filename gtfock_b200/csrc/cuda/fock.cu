@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "devmem.cuh"
+#include "gtf_basis.h"
 #include "gtf_cuda.h"
 #include "gtf_dev.cuh"
 #include "sph_dev.cuh"
@@ -748,7 +749,7 @@ __global__ void k_build_pairs(const int *__restrict__ idx, const int *__restrict
 // them (one thread sorting up to 64 records in global memory by insertion
 // took 1.5 ms for C12H26 / cc-pVDZ).
 #define FILL_WARPS 4
-#define FILL_MAX 256   // primitive pairs kept in shared memory; the rest are evaluated again for each rank
+#define FILL_MAX (GTF_MAX_NPRIM * GTF_MAX_NPRIM)
 __global__ void __launch_bounds__(32 * FILL_WARPS)
     k_fill_primpairs(PairRec *__restrict__ pairs, const int *__restrict__ idx, const int *__restrict__ shellid,
                      const int *__restrict__ shellrid, const int *__restrict__ pair_off, BasisDev b, int npairs,
@@ -767,11 +768,10 @@ __global__ void __launch_bounds__(32 * FILL_WARPS)
     const double r2 = (Ax - Bx) * (Ax - Bx) + (Ay - By) * (Ay - By) + (Az - Bz) * (Az - Bz);
     const int nb = b.sh_nprim[bb], n = b.sh_nprim[a] * nb;
     const int pa = b.sh_pstart[a], pb = b.sh_pstart[bb];
-    auto abs_k = [&](int q) {
+    for (int q = lane; q < n; q += 32) {
         double p;
-        return fabs(prim_pair_K(b, pa, pb, q / nb, q % nb, r2, p));
-    };
-    for (int q = lane; q < n && q < FILL_MAX; q += 32) sh[w][q] = abs_k(q);
+        sh[w][q] = fabs(prim_pair_K(b, pa, pb, q / nb, q % nb, r2, p));
+    }
     __syncwarp();
     constexpr int W = 2 * GTF_PPREC_D2;
     int kept = 0;
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(32 * FILL_WARPS)
         kept++;
         int o = 0;
         for (int t = 0; t < n; t++) {
-            const double u = t < FILL_MAX ? sh[w][t] : abs_k(t);
+            const double u = sh[w][t];
             if (u >= GTF_PRIM_EPS && (u > v || (u == v && t < q))) o++;
         }
         const double al = b.alpha[pa + i], be = b.alpha[pb + j], ip = 1.0 / p;
@@ -2178,9 +2178,10 @@ static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *F
 // Builds of at most this many units (32 lanes each) over all launches run
 // them over several streams.  A launch of a small molecule occupies a few SMs
 // for the latency of its longest lane, and up to 62 of them (124 in mixed
-// precision) in a row add up.  Above, one launch fills the GPU: overlapping
-// tails gained at most 1.6% on C54H18 / cc-pVDZ (13.4M units) and (H2O)64 /
-// 6-31G (9.8M), and the times per class pair would no longer add up.
+// precision) in a row add up (ethane / cc-pVDZ 2.0 -> 0.47 ms, C12H26 8.9 ->
+// 7.7 ms).  Above, one launch fills the GPU: overlapping tails gained at most
+// 0.5% on C54H18 / cc-pVDZ (13.4M units) and (H2O)64 / 6-31G (9.8M), and the
+// times per class pair would no longer add up.
 #define GTF_OVERLAP_UNITS 2000000LL
 
 // All class pairs of one build; timed: events around each; may_create: the

@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
     constexpr int S = fock_slice(LA, LB, LC, LD, sizeof(R) == 4 ? 1 : 0);
     constexpr int N = (NCD - CD0 < S) ? NCD - CD0 : S;
     constexpr bool LOW = low_class(LA, LB, LC, LD);
-    __shared__ __align__(16) R tab[LOW ? BoysTab<R>::LEN : RysTab<R>::len(NR)];
+    __shared__ __align__(16) R tab[LOW ? BoysTab<R>::LEN : RysTab<R>::slen(NR)];
     // the launch's unit count, kept in shared memory rather than a register
     // across the integral loops (visible after the staging's barrier)
     __shared__ unsigned long long s_nunits;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
     if constexpr (LOW) {
         table_stage<BoysTab<R>::LEN>(tab, BoysTab<R>::ptr(LA + LB + LC + LD));
     } else {
-        table_stage<RysTab<R>::len(NR)>(tab, RysTab<R>::ptr(NR));
+        rys_stage<R, NR>(tab);
     }
     const int lane = threadIdx.x & 31;
     // batched launches: per-warp slots for the claimed range of units and the
@@ -285,10 +285,10 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
         for (int k = 0; k < ncart(LA) * ncart(LB) * N; k++) acc[k] = (R)0;
         if constexpr (sizeof(R) == 4) {
             const PPRec32 src{GTF_FLD(pprec32)};
-            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true, LOW>(src, pb, pk, acc, tab, split);
+            if (active) eri_accumulate_cd32<LA, LB, LC, LD, CD0, N, true, true, LOW>(src, pb, pk, acc, tab, split);
         } else {
             const PPRec src{GTF_FLD(pprec)};
-            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true, LOW>(src, pb, src, pk, acc, tab, split);
+            if (active) eri_accumulate_cd<LA, LB, LC, LD, CD0, N, true, true, LOW>(src, pb, src, pk, acc, tab, split);
         }
         // sum the lanes of each quartet; the first of them digests it
         const int nl = (split & 0xff) * ((split >> 8) & 0xff);

@@ -139,10 +139,12 @@ __host__ __device__ constexpr int rys_deg(int n)
 }
 
 // The N-root block of each table is [off(N), off(N+1)); its extent is known
-// at compile time so kernels can stage it in shared memory.  An interval is
-// stride(N) values of pairs (u_r, w_r), an odd number of pairs (16 bytes FP64,
-// 8 bytes FP32): the lanes of a warp read different intervals, and
-// consecutive ones then start in different banks.
+// at compile time so kernels can stage it in shared memory.  rows(N) values
+// per interval.  The shared-memory copy has pairs (u_r, w_r), so that one
+// vector load serves a step of both polynomials, and srows(N) values per
+// interval, an odd number of pairs (16 bytes FP64, 8 bytes FP32): the lanes
+// of a warp read different intervals, and consecutive ones then start in
+// different banks.
 template <typename R>
 struct RysTab;
 template <>
@@ -156,7 +158,9 @@ struct RysTab<double> {
     static __host__ __device__ constexpr int len(int n) { return off(n + 1) - off(n); }
     static __host__ __device__ constexpr int deg(int n) { return rys_deg(n); }
     static __host__ __device__ constexpr double h(int n) { return rys_h(n); }
-    static __host__ __device__ constexpr int stride(int n) { return 2 * ((deg(n) + 1) * n | 1); }
+    static __host__ __device__ constexpr int rows(int n) { return 2 * (deg(n) + 1) * n; }
+    static __host__ __device__ constexpr int srows(int n) { return 2 * ((deg(n) + 1) * n | 1); }
+    static __host__ __device__ constexpr int slen(int n) { return len(n) / rows(n) * srows(n); }
     static __device__ __forceinline__ const double *ptr(int n) { return RYS_TABLE + off(n); }
 };
 template <>
@@ -170,14 +174,16 @@ struct RysTab<float> {
     static __host__ __device__ constexpr int len(int n) { return off(n + 1) - off(n); }
     static __host__ __device__ constexpr int deg(int) { return RYS32_DEG; }
     static __host__ __device__ constexpr float h(int) { return (float)RYS32_H; }
-    static __host__ __device__ constexpr int stride(int n) { return 2 * ((deg(n) + 1) * n | 1); }
+    static __host__ __device__ constexpr int rows(int n) { return 2 * (deg(n) + 1) * n; }
+    static __host__ __device__ constexpr int srows(int n) { return 2 * ((deg(n) + 1) * n | 1); }
+    static __host__ __device__ constexpr int slen(int n) { return len(n) / rows(n) * srows(n); }
     static __device__ __forceinline__ const float *ptr(int n) { return RYS32_TABLE + off(n); }
 };
 
-// Stages LEN values of a table into shared memory: 16-byte asynchronous copies,
-// all in flight at once.  (A loop of 8-byte loads was one dependent round
-// trip to L2 per thread and pass, up to 46 of them: most of the time of a
-// launch with little work.)
+// Stages LEN values of a table into shared memory: 16-byte asynchronous
+// copies, all in flight at once.  (A loop of dependent 8-byte loads, up to 46
+// round trips to L2 per thread, was most of the time of a launch with little
+// work.)
 template <int LEN, typename R>
 __device__ __forceinline__ void table_stage(R *stab, const R *table)
 {
@@ -191,12 +197,27 @@ __device__ __forceinline__ void table_stage(R *stab, const R *table)
     __syncthreads();
 }
 
+// Stages the N-root block with its values paired, eight loads in flight.
+template <typename R, int N>
+__device__ __forceinline__ void rys_stage(R *stab)
+{
+    constexpr int RW = RysTab<R>::rows(N), SR = RysTab<R>::srows(N), TL = RysTab<R>::len(N);
+    static_assert(TL % RW == 0, "whole intervals");
+    const R *gt = RysTab<R>::ptr(N);
+#pragma unroll 8
+    for (int k = threadIdx.x; k < TL; k += blockDim.x) {
+        const int row = k / RW, e = k % RW, j = e / (2 * N), q = e % (2 * N);
+        stab[row * SR + j * 2 * N + (q < N ? 2 * q : 2 * (q - N) + 1)] = __ldg(gt + k);
+    }
+    __syncthreads();
+}
+
 // Roots and weights of one argument T: below RYS_TMAX the interval's
 // polynomials in s (a degree-7 fit in FP32, the FP64 table's degrees
 // otherwise), above it the large-T form.  tab: the N-root block of the global
-// table or its copy in shared memory.  all() evaluates every root at once,
-// root() one of them.
-template <int N, typename R>
+// table, or (PAIRED) its copy in shared memory.  all() evaluates every root at
+// once, root() one of them.
+template <int N, bool PAIRED, typename R>
 struct RysArg {
     R a, b;         // s and -, or 1/T and 1/sqrt(T)
     const R *row;   // the interval's coefficients; null: large T
@@ -211,7 +232,19 @@ struct RysArg {
             const int k = (int)(T * INV_H);
             a = T - ((R)k * H + (R)0.5 * H);
             b = (R)0;
-            row = tab + k * RysTab<R>::stride(N);
+            row = tab + k * (PAIRED ? RysTab<R>::srows(N) : RysTab<R>::rows(N));
+        }
+    }
+    // coefficient j of root r and of its weight
+    __device__ __forceinline__ void coef(int j, int r, R &u, R &w) const
+    {
+        if constexpr (PAIRED) {
+            const typename RysTab<R>::V2 t = reinterpret_cast<const typename RysTab<R>::V2 *>(row)[j * N + r];
+            u = t.x;
+            w = t.y;
+        } else {
+            u = row[j * 2 * N + r];
+            w = row[j * 2 * N + N + r];
         }
     }
     __device__ __forceinline__ void all(R (&u)[N], R (&w)[N]) const
@@ -225,21 +258,16 @@ struct RysArg {
             }
             return;
         }
-        typedef typename RysTab<R>::V2 V2;
-        const V2 *c2 = reinterpret_cast<const V2 *>(row);
 #pragma unroll
-        for (int i = 0; i < N; i++) {
-            const V2 t = c2[DEG * N + i];
-            u[i] = t.x;
-            w[i] = t.y;
-        }
+        for (int i = 0; i < N; i++) coef(DEG, i, u[i], w[i]);
 #pragma unroll
         for (int j = DEG - 1; j >= 0; j--) {
 #pragma unroll
             for (int i = 0; i < N; i++) {
-                const V2 t = c2[j * N + i];
-                u[i] = gfma(u[i], a, t.x);
-                w[i] = gfma(w[i], a, t.y);
+                R tu, tw;
+                coef(j, i, tu, tw);
+                u[i] = gfma(u[i], a, tu);
+                w[i] = gfma(w[i], a, tw);
             }
         }
     }
@@ -251,16 +279,13 @@ struct RysArg {
             w = (R)RYS_LARGE_W[N][r] * b;
             return;
         }
-        typedef typename RysTab<R>::V2 V2;
-        const V2 *c2 = reinterpret_cast<const V2 *>(row) + r;
-        const V2 t0 = c2[DEG * N];
-        u = t0.x;
-        w = t0.y;
+        coef(DEG, r, u, w);
 #pragma unroll
         for (int j = DEG - 1; j >= 0; j--) {
-            const V2 t = c2[j * N];
-            u = gfma(u, a, t.x);
-            w = gfma(w, a, t.y);
+            R tu, tw;
+            coef(j, r, tu, tw);
+            u = gfma(u, a, tu);
+            w = gfma(w, a, tw);
         }
     }
 };
@@ -370,13 +395,14 @@ __host__ __device__ constexpr int prim_split(int ks, int k0, int bs, int b0)
 // call it once per slice so that a slice's accumulators fit in registers.
 // R = double, or float for quartets evaluated in single precision (the
 // differences of centres are formed in double first, then rounded).
+// SPAD: rtab is the paired copy in shared memory (rys_stage).
 // LOW: Boys functions and recurrences (eri_low.cuh) instead of Rys quadrature;
 // rtab is then the F_m rows of BOYS_TABLE, m the total angular momentum.
 // rtab: the NR-root block of the Rys table of precision R.
 // Loop order: ket primitive pairs outside (one per lane), bra primitive pairs
 // inside -- the bra is shared by the warp, so its records are warp-uniform
 // loads that stay in L1, and each lane reads its ket's records once.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool LOW = false, class PPB, class PPK,
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool SPAD = false, bool LOW = false, class PPB, class PPK,
           typename R>
 __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec &pb, const PPK &ket,
                                                   const PairRec &pk, R (&acc)[ncart(LA) * ncart(LB) * N],
@@ -417,7 +443,7 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
                 low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (R)0.5 * ipq);
                 continue;
             }
-            const RysArg<NR, R> rys(T, rtab);
+            const RysArg<NR, SPAD, R> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             R u[NR], w[NR];
             if constexpr (!LOOP) rys.all(u, w);
@@ -474,7 +500,7 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
 // FP32 quartets: everything in single precision, from the FP32 records (centres
 // relative to each pair's first shell; P - Q = PA - QC + (A - C) with A - C
 // formed in double once per quartet).  Same structure as eri_accumulate_cd.
-template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool LOW = false>
+template <int LA, int LB, int LC, int LD, int CD0, int N, bool SKIP, bool SPAD = false, bool LOW = false>
 __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const PairRec &pb, const PairRec &pk,
                                                     float (&acc)[ncart(LA) * ncart(LB) * N], const float *rtab,
                                                     int split = prim_split(1, 0, 1, 0))
@@ -515,7 +541,7 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
                 low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (float)0.5 * ipq);
                 continue;
             }
-            const RysArg<NR, float> rys(T, rtab);
+            const RysArg<NR, SPAD, float> rys(T, rtab);
             constexpr bool LOOP = rys_loop(LA + LB);
             float u[NR], w[NR];
             if constexpr (!LOOP) rys.all(u, w);

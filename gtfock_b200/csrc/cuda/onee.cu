@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128)
             }
             const double T = p * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
             double u[NR], wt[NR];
-            RysArg<NR, double>(T, RysTab<double>::ptr(NR)).all(u, wt);
+            RysArg<NR, false, double>(T, RysTab<double>::ptr(NR)).all(u, wt);
             const double pref = -(double)Z[c] * 2.0 * M_PI * ip * K;
 #pragma unroll
             for (int r = 0; r < NR; r++) {

@@ -156,21 +156,6 @@ def fmt(x, single=False):
     return "%.17e" % float(x)
 
 
-def layout(intervals, n, deg, align):
-    """One root count's intervals, flat: per interval and coefficient the pairs
-    (u_r, w_r), a pair of zeros where the interval would have an even number
-    of pairs (the interval stride of kernels that stage the block in shared
-    memory, free of bank conflicts), and zeros up to a multiple of `align`."""
-    flat = []
-    for iv in intervals:
-        for j in range(deg + 1):
-            for r in range(n):
-                flat += [iv[r][j], iv[n + r][j]]
-        if (deg + 1) * n % 2 == 0:
-            flat += [0, 0]
-    return flat + [0] * (-len(flat) % align)
-
-
 def main(out_path=None):
     if out_path is None:
         out_path = os.path.join(os.path.dirname(os.path.abspath(__file__)),
@@ -186,11 +171,10 @@ def main(out_path=None):
     w("/* rys_table.h -- generated by gtfock_b200/gen_rys_table.py; do not edit.")
     w(" * Rys quadrature for the Boys weight: per root count n, per interval of")
     w(" * width H_n in T (RYS_H_LIST), DEG_n+1 monomial coefficients (RYS_DEG_LIST)")
-    w(" * in s = T - (T0 + H_n/2), stored [interval][coef][root] as pairs (u, w),")
-    w(" * every interval an odd number of pairs long and every n's block a multiple")
-    w(" * of 16 bytes (zero padding); above RYS_TMAX[n] the Hermite large-T form")
+    w(" * in s = T - (T0 + H_n/2) for u_1..u_n then w_1..w_n, stored")
+    w(" * [interval][coef][func]; above RYS_TMAX[n] the Hermite large-T form")
     w(" * u = x^2/T, w = W/sqrt(T) applies.  The FP32 table uses RYS32_H and")
-    w(" * RYS32_DEG for every n. */")
+    w(" * RYS32_DEG for every n.  BOYS_TABLE, BOYS32_TABLE: see the generator. */")
     w("#pragma once")
     w("#ifndef RYS_QUAL")
     w("#define RYS_QUAL static")
@@ -208,7 +192,7 @@ def main(out_path=None):
     flat = []
     for n in range(1, NMAX + 1):
         offs[n] = len(flat)
-        flat += layout(t64[n], n, DEG64[n], 2)
+        flat += [iv[f][j] for iv in t64[n] for j in range(DEG64[n] + 1) for f in range(2 * n)]
     w("RYS_QUAL_SMALL const double RYS_TMAX[RYS_NMAX + 1] = {0.0, %s};" %
       ", ".join("%.1f" % TMAX[n] for n in range(1, NMAX + 1)))
     w("RYS_QUAL_SMALL const int RYS_OFF[RYS_NMAX + 1] = {0, %s};" %
@@ -223,7 +207,7 @@ def main(out_path=None):
     flat32 = []
     for n in range(1, NMAX + 1):
         offs32[n] = len(flat32)
-        flat32 += layout(t32[n], n, DEG32, 4)
+        flat32 += [iv[f][j] for iv in t32[n] for j in range(DEG32 + 1) for f in range(2 * n)]
     w("RYS_QUAL_SMALL const int RYS32_OFF[RYS_NMAX + 1] = {0, %s};" %
       ", ".join(str(offs32[n]) for n in range(1, NMAX + 1)))
     w("#define RYS32_OFF_LIST 0, %s" % ", ".join(str(offs32[n]) for n in range(1, NMAX + 1)))
