@@ -103,6 +103,9 @@ struct FockGrid {
     // a warp claims at once
     int ctas_per_sm;
     int claim;
+    // one-molecule launches: units a block claims in a row (0: every warp
+    // claims its own; GTF_CHUNK_ROUNDS)
+    int chunk;
     int query;                      // launch nothing: return the first slice's occupancy limit
     // single-molecule launches of a sharded build: this launch covers units
     // [unit_lo, unit_lo + nunits) of the class's unit range
@@ -183,7 +186,19 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
     // the launch's unit count, kept in shared memory rather than a register
     // across the integral loops (visible after the staging's barrier)
     __shared__ unsigned long long s_nunits;
-    if (threadIdx.x == 0) s_nunits = (unsigned long long)(g.nunits_dev ? *g.nunits_dev : g.nunits);
+    // the block's pool of claimed units: (next unit) << 16 | units left
+    __shared__ unsigned long long s_pool;
+    auto claim_chunk = [&]() {
+        const unsigned long long c = atomicAdd(counter, (unsigned long long)g.chunk);
+        const unsigned long long n = *(volatile unsigned long long *)&s_nunits;
+        const unsigned long long left = c >= n ? 0 : n - c < (unsigned long long)g.chunk ? n - c : g.chunk;
+        atomicExch(&s_pool, c << 16 | left);
+    };
+    if (threadIdx.x == 0) {
+        s_nunits = (unsigned long long)(g.nunits_dev ? *g.nunits_dev : g.nunits);
+        s_pool = 0;
+        if (!BATCH && g.chunk > 0) claim_chunk();
+    }
     if constexpr (LOW) {
         table_stage<BoysTab<R>::LEN>(tab, BoysTab<R>::ptr(LA + LB + LC + LD));
     } else {
@@ -228,7 +243,20 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
             __syncwarp();
         } else {
             unsigned long long c0 = 0;
-            if (lane == 0) c0 = atomicAdd(counter, 1ULL);
+            if (lane == 0) {
+                // from the block's pool; whoever takes its last unit claims
+                // the next chunk, and a warp that finds it empty meanwhile
+                // claims one unit for itself
+                unsigned long long v = g.chunk > 0 ? *(volatile unsigned long long *)&s_pool : 0;
+                while ((v & 0xffff) != 0) {
+                    const unsigned long long o = atomicCAS(&s_pool, v, v + 0xffff);   // next + 1, left - 1
+                    if (o == v) break;
+                    v = o;
+                }
+                if ((v & 0xffff) == 0) c0 = atomicAdd(counter, 1ULL);
+                else c0 = v >> 16;
+                if ((v & 0xffff) == 1) claim_chunk();
+            }
             uu = __shfl_sync(GTF_FULL_MASK, c0, 0);
             if (uu >= *(volatile unsigned long long *)&s_nunits) break;
             uu = *(volatile unsigned long long *)&s_nunits - 1 - uu + (unsigned long long)g.unit_lo;
@@ -311,6 +339,13 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
 // Units per resident warp from which a launch uses one large block per SM.
 #define GTF_BIG_ROUNDS 4
 
+// From GTF_CHUNK_ROUNDS units per resident warp on, a block claims chunks of
+// two units per warp for all its warps: they then work on the same bra, whose
+// rows of D stay in the SM's L1.  (Chunks dealt to the blocks in turn, without
+// the counter, were as good for (H2O)64 but left C54H18's blocks unbalanced:
+// 190 ms against 182.)  Below, single units balance better.
+#define GTF_CHUNK_ROUNDS 16
+
 // Streams the launches of a build are dealt out to in turn (n == 1: all in
 // order on one stream).
 #define GTF_FOCK_STREAMS 8
@@ -364,7 +399,10 @@ int launch_fock_slices(const FockGrid &g, FockStreams &st, int slice)
         long long grid = (long long)g.nsm * per_sm;
         if (want < grid) grid = want;
         if (grid < 1) grid = 1;
-        k<<<(unsigned)grid, threads, 0, st.take()>>>(g, g.counter + slice);
+        FockGrid gl = g;
+        if (g.nmol <= 1 && threads == BIG && g.nunits >= (long long)g.nsm * (BIG / 32) * GTF_CHUNK_ROUNDS)
+            gl.chunk = 2 * (BIG / 32);
+        k<<<(unsigned)grid, threads, 0, st.take()>>>(gl, g.counter + slice);
         if (cudaGetLastError() != cudaSuccess) return -1;
         const int r = launch_fock_slices<LA, LB, LC, LD, R, CD0 + S>(g, st, slice + 1);
         return r < 0 ? r : r + 1;
