@@ -9,7 +9,8 @@
 //     quadrature -- per primitive quartet and root the 2-D integrals
 //     G(i,k) by the Rys recurrences (C00, C00', B10, B01, B00), horizontal
 //     transfer to (a b | c d) per Cartesian direction, and the product
-//     Ix*Iy*Iz accumulated in registers; integrals never leave the thread;
+//     Ix*Iy*Iz accumulated in registers; integrals never leave the thread
+//     (classes of small total angular momentum: eri_low.cuh);
 //   * digest_cd<...>: the six J/K updates of one unique quartet into F with
 //     the reference's degeneracy factors; the bra block (uniform across a
 //     warp) is warp-reduced before its atomics.

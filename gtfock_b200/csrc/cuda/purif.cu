@@ -1,5 +1,6 @@
 // purif.cu -- canonical density purification and Pulay DIIS on one GPU
-// (pscf/purif.c:257-641; the 3-D pdgemm of pscf/pdgemm.c becomes one DGEMM).
+// (pscf/purif.c:257-641; the 3-D pdgemm of pscf/pdgemm.c becomes one product:
+// k_sym_abt for the symmetric ones, cuBLAS DGEMM for the others).
 //
 // Purification (pscf/purif.c:301-476): Gershgorin bounds and tr F give the
 // initial D; each iteration forms D2 = D D^T and D3 = D D2, reduces
@@ -7,7 +8,7 @@
 // partials summed in order), updates D with the trace-conserving polynomial,
 // and stops once ||D - D2||_F < 1e-11.  D_AO = X D X at the end.
 // DIIS (pscf/purif.c:491-641): error X (F D S - S D F) X, dot products into
-// the bordered B matrix, (m+1)^2 solve on the host, F = sum c_i F_i.
+// the bordered B matrix, (m+1)^2 solve, F = sum c_i F_i.
 #include <cublas_v2.h>
 #include <cuda_runtime.h>
 #include <float.h>
