@@ -116,8 +116,7 @@ struct ClassPairTask {
 // join() lets fs.s[0] go on once they are through.  The sets come from a
 // process-wide pool (creating one takes 0.3 ms) and return to it with the
 // engine or batch that took them, at most GTF_SIDE_SETS waiting there; a set
-// that returns has been joined, so whoever takes it next only queues behind
-// work that its former owner has waited for.
+// that returns has been waited for.
 #define GTF_SIDE_SETS 16
 struct SideStreams {
     int dev;
@@ -187,6 +186,8 @@ struct ForkJoin {
     void give_back()
     {
         if (!p) return;
+        // a build that failed between fork and join left work unjoined
+        for (cudaStream_t q : p->s) cudaStreamSynchronize(q);
         {
             std::lock_guard<std::mutex> lk(g_side_mu);
             if (g_side.size() < GTF_SIDE_SETS) {
