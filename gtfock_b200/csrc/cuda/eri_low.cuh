@@ -16,8 +16,8 @@
 // the recurrences take fewer operations than the products of the 2-D integrals.
 #pragma once
 
-// F_0 .. F_m of the table's intervals: row of polynomial coefficients of F_m
-// in s = T - T_mid, then exp(-T_mid)
+// H_m = F_m / (2m - 1)!! on the table's intervals: row of polynomial
+// coefficients in s = T - T_mid, then exp(-T_mid)
 template <typename R>
 struct BoysTab;
 template <>
@@ -41,14 +41,21 @@ struct BoysTab<float> {
     }
 };
 
-// F[0..M] at T; row0: the F_M rows (global or shared).  Above BOYS_TMAX exp(-T) is below the rounding of every F_m, m <= 4.
+// (2m - 1)!!, m <= 4 (no recursion: it must fold in the unrolled loops)
+__host__ __device__ constexpr double boys_dfac(int m) { return m <= 1 ? 1.0 : m == 2 ? 3.0 : m == 3 ? 15.0 : 105.0; }
+
+// F[0..M] at T; row0: the rows of H_M (global or shared).  Above BOYS_TMAX
+// exp(-T) is below the rounding of every F_m, m <= 4.  Within 3 units in the
+// last place below it; above, the rounding of 1 / T enters F_m m times.
 template <int M, typename R>
 __device__ __forceinline__ void boys(R T, R (&F)[M + 1], const R *row0)
 {
     typedef BoysTab<R> Tab;
     static_assert(M <= BOYS_MMAX, "table");
     if (T >= (R)BOYS_TMAX) {
-        const R rs = grsqrt(T), it = rs * rs;
+        const R rs = grsqrt(T);
+        R it = rs * rs;
+        it = gfma(it, gfma(-T, it, (R)1), it);   // 1 / T: one Newton step takes rsqrt's rounding out
         F[0] = (R)0.886226925452758014 * rs;   // sqrt(pi) / 2
 #pragma unroll
         for (int m = 0; m < M; m++) F[m + 1] = F[m] * ((R)(m + 0.5) * it);
@@ -57,20 +64,20 @@ __device__ __forceinline__ void boys(R T, R (&F)[M + 1], const R *row0)
     const int k = (int)(T * (R)(1.0 / BOYS_H));
     const R s = T - ((R)k * (R)BOYS_H + (R)(0.5 * BOYS_H));
     const R *c = row0 + k * Tab::ROW;
-    R f = c[Tab::DEG];
+    R h = c[Tab::DEG];
 #pragma unroll
-    for (int j = Tab::DEG - 1; j >= 0; j--) f = gfma(f, s, c[j]);
-    F[M] = f;
+    for (int j = Tab::DEG - 1; j >= 0; j--) h = gfma(h, s, c[j]);
+    F[M] = M > 1 ? h * (R)boys_dfac(M) : h;
     if constexpr (M > 0) {
-        R e = Tab::ecoef(Tab::EDEG);
+        R q = Tab::ecoef(Tab::EDEG);
 #pragma unroll
-        for (int j = Tab::EDEG - 1; j >= 0; j--) e = gfma(e, s, Tab::ecoef(j));
-        e *= c[Tab::DEG + 1];
+        for (int j = Tab::EDEG - 1; j >= 0; j--) q = gfma(q, s, Tab::ecoef(j));
+        const R E = c[Tab::DEG + 1], e = gfma(E * s, q, E);
         const R t2 = (R)2 * T;
 #pragma unroll
         for (int m = M; m > 0; m--) {
-            const R v = gfma(t2, F[m], e);
-            F[m - 1] = m == 1 ? v : v * (R)(1.0 / (2 * m - 1));
+            h = gfma(t2, h, m > 1 ? e * (R)(1.0 / boys_dfac(m)) : e);
+            F[m - 1] = m > 2 ? h * (R)boys_dfac(m - 1) : h;
         }
     }
 }

@@ -20,10 +20,11 @@ Method (published, restated here):
     u_i = x_i^2 / T, w_i = W_i / sqrt(T) with x_i > 0 the roots of the Hermite
     polynomial H_2n and W_i their Gauss-Hermite weights.
 The light classes (total angular momentum up to 4) need only Boys functions
-F_0 .. F_m: per m and interval of width HB a polynomial for F_m and exp(-T) at
-the middle; exp(-T) elsewhere in the interval is that times a polynomial for
-exp(-s), and F_m-1 .. F_0 follow by the downward recursion
-F_k-1 = (2 T F_k + exp(-T)) / (2k - 1).
+F_0 .. F_m, as H_k = F_k / (2k - 1)!!: per m and interval of width HB a
+polynomial for H_m and E = exp(-T) at the middle; exp(-T) elsewhere in the
+interval is E + E s q(s) with a polynomial q for (exp(-s) - 1) / s, and
+H_m-1 .. H_0 follow by the downward recursion
+H_k-1 = 2 T H_k + exp(-T) / (2k - 1)!!, in which no step divides.
 Accuracy of the double table against the 60-digit values: <= 1e-15 relative
 (checked by tests/test_oracle.py against values recomputed here).
 
@@ -46,12 +47,12 @@ TMAX = {1: 40.0, 2: 48.0, 3: 56.0, 4: 62.0, 5: 70.0}
 # single-precision table for the mixed-precision kernels
 H32 = 2.0
 DEG32 = 7
-# Boys functions: interval width, range, degrees of F_m and of exp(-s)
+# Boys functions: interval width, range, degrees of F_m and of (exp(-s) - 1) / s
 HB = 0.5
 TB = 48.0
 BMAX = 4
 DEGB = {64: 9, 32: 5}
-DEGE = {64: 10, 32: 5}
+DEGE = {64: 9, 32: 4}
 DPS = 60
 
 
@@ -133,8 +134,8 @@ def fit_boys(args):
     m, k, deg = args
     with mp.workdps(DPS):
         mid = mp.mpf((k + 0.5) * HB)
-        return chebyshev_fit(lambda s: boys_moments(mid + s, 2)[0] if m == 0 else
-                             mp.hyp1f1(m + mp.mpf(1) / 2, m + mp.mpf(3) / 2, -(mid + s)) / (2 * m + 1),
+        scale = (2 * m + 1) * mp.fac2(2 * m - 1)
+        return chebyshev_fit(lambda s: mp.hyp1f1(m + mp.mpf(1) / 2, m + mp.mpf(3) / 2, -(mid + s)) / scale,
                              HB, deg) + [mp.exp(-mid)]
 
 
@@ -228,7 +229,7 @@ def main(out_path=None):
     for n in range(1, NMAX + 1):
         w("  {" + ", ".join(fmt(wt) for _, wt in hl[n]) + "},")
     w("};")
-    # Boys functions: [m][interval][coefficients of F_m, exp(-T_mid)]
+    # Boys functions: [m][interval][coefficients of F_m / (2m - 1)!!, exp(-T_mid)]
     w("#define BOYS_MMAX %d" % BMAX)
     w("#define BOYS_H %.1f" % HB)
     w("#define BOYS_TMAX %.1f" % TB)
@@ -237,7 +238,7 @@ def main(out_path=None):
         w("#define %s_DEG %d" % (name, DEGB[p]))
         w("#define %s_EXP_DEG %d" % (name, DEGE[p]))
         w("#define %s_EXP_LIST %s" % (name, ", ".join(
-            fmt(c, p == 32) for c in chebyshev_fit(lambda s: mp.exp(-s), mp.mpf(HB), DEGE[p]))))
+            fmt(c, p == 32) for c in chebyshev_fit(lambda s: mp.expm1(-s) / s if s else mp.mpf(-1), mp.mpf(HB), DEGE[p]))))
         vals = [c for m in range(BMAX + 1) for row in boys[p][m] for c in row]
         w("RYS_QUAL const %s %s_TABLE[%d] = {" % (typ, name, len(vals)))
         for i in range(0, len(vals), 4):
