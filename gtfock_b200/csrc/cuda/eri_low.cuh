@@ -3,17 +3,28 @@
 // gtf_dev.cuh.
 //
 // (ss|ss) (ps|ss) (ps|ps) (pp|ss) (ds|ss) (ds|ps) (pp|ps) (dp|ss), most of a
-// build's quartets, and (dp|ps) (ds|pp) (ds|ds) (dd|ss).  Per primitive quartet, with S_m = pref F_m(T), the
-// Obara-Saika recurrences (S. Obara, A. Saika, J. Chem. Phys. 84, 3963 (1986))
-// build only (a s|c s); (pp|, (dp| and (dd| follow from these by
-// the horizontal transfer (a b+1| = (a+1 b| + (A - B)(a b|, which does not
-// depend on the primitives and is applied once, to the contracted sums.
+// build's quartets, and (dp|ps) (ds|pp) (ds|ds) (dd|ss).  Per primitive
+// quartet, with S_m = pref F_m(T), the Obara-Saika recurrences (S. Obara,
+// A. Saika, J. Chem. Phys. 84, 3963 (1986)) raise every index about its own
+// centre.
 //
 // Why: the Rys kernels of these classes kept the L1 pipe 65-81% busy and the
 // FP64 pipe below 50%: each primitive quartet read 10 pairs of 16 bytes per
 // root from the table in shared memory.  One Boys polynomial and one
 // exponential read 88 bytes whatever the class, from a table of 8 KB, and
 // the recurrences take fewer operations than the products of the 2-D integrals.
+//
+// Accuracy: over random contracted quartets (tests/host/eri_accuracy.cpp) the
+// error relative to a quartet's largest integral is 0.7 to 1.0 times that of
+// the Rys form in FP64 and in FP32, for two reasons.  (pp|, (dp|, (dd| and |pp)
+// are raised with P - B (Q - D); moving the second index by the horizontal
+// transfer (a b+1| = (a+1 b| + (A - B)(a b|, on the contracted sums, cancels
+// where P is close to B: 1.3 to 2.8 times the error of the Rys form.  And the
+// last step to an integral is summed before it is added to acc, one rounding
+// of the contracted sum instead of one per term (1.0 to 1.2 times otherwise),
+// but for (ds|pp) and (dd|ss), which stay below 1.0 without and whose sums
+// fill the registers.  C54H18 / cc-pVDZ: 181.2 ms against 176.4 with the
+// transfer, (H2O)64 / 6-31G 30.0 against 29.7.
 #pragma once
 
 // H_m = F_m / (2m - 1)!! on the table's intervals: row of polynomial
@@ -89,42 +100,24 @@ __host__ __device__ constexpr bool low_class(int LA, int LB, int LC, int LD)
     return LA + LB + LC + LD <= 3 || (LA + LB + LC + LD == 4 && !(LA == 1 && LB == 1));
 }
 
-// index of the d component ij and of the f component ijk (x = 0, y = 1, z = 2):
-// with ny and nz of its factors y and z, (ny + nz)(ny + nz + 1) / 2 + nz
+// index of the d component ij (x = 0, y = 1, z = 2): with ny and nz of its
+// factors y and z, (ny + nz)(ny + nz + 1) / 2 + nz
 __host__ __device__ constexpr int cart_of(int ny, int nz) { return (ny + nz) * (ny + nz + 1) / 2 + nz; }
 __host__ __device__ constexpr int d_of(int i, int j) { return cart_of((i == 1) + (j == 1), (i == 2) + (j == 2)); }
-__host__ __device__ constexpr int f_of(int i, int j, int k)
-{
-    return cart_of((i == 1) + (j == 1) + (k == 1), (i == 2) + (j == 2) + (k == 2));
-}
 
-// index of the g component ijkl
-__host__ __device__ constexpr int g_of(int i, int j, int k, int l)
-{
-    return cart_of((i == 1) + (j == 1) + (k == 1) + (l == 1), (i == 2) + (j == 2) + (k == 2) + (l == 2));
-}
-
-// contracted sums the primitive loops keep: the (a s|c s) with a from LA to
-// LA + LB (all three of (dd|) on LC + LD, for (ds|pp) also on LC
-__host__ __device__ constexpr int low_nsum(int LA, int LB, int LC, int LD)
-{
-    const int l = LA + LB;
-    if (LC + LD == 2) return ncart(l) * (ncart(2) + (LD == 1 ? ncart(1) : 0));
-    int n = 0;
-    for (int a = LA; a <= l; a++) n += ncart(a) * ncart(LC);
-    return n;
-}
-
-// one primitive quartet: S[m] = pref F_m, m <= LA + LB + LC + LD
+// adds one primitive quartet to acc[ia + NA*(ib + NB*(ic + NC*id))]:
+// S[m] = pref F_m, m <= LA + LB + LC + LD
 template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void low_prim(R (&v)[low_nsum(LA, LB, LC, LD)], const R (&S)[LA + LB + LC + LD + 1],
-                                         const R (&PA)[3], const R (&QC)[3], const R (&PQ)[3], R qf, R pf, R h2p,
+__device__ __forceinline__ void low_prim(R (&v)[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)],
+                                         const R (&S)[LA + LB + LC + LD + 1], const R (&PA)[3], const R (&AB)[3],
+                                         const R (&QC)[3], const R (&CD)[3], const R (&PQ)[3], R qf, R pf, R h2p,
                                          R h2q, R hpq)
 {
     constexpr int L = LA + LB, LT = L + LC + LD;
     if constexpr (LT == 0) {
         v[0] += S[0];
     } else {
+        // (ps|ss)^m
         R WP[3], P[LT][3];
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -132,9 +125,17 @@ __device__ __forceinline__ void low_prim(R (&v)[low_nsum(LA, LB, LC, LD)], const
 #pragma unroll
             for (int m = 0; m < LT; m++) P[m][i] = gfma(PA[i], S[m], WP[i] * S[m + 1]);
         }
-        R WQ[3];
+        R WQ[3], PB[3], QD[3];
 #pragma unroll
-        for (int k = 0; k < 3; k++) WQ[k] = pf * PQ[k];
+        for (int k = 0; k < 3; k++) {
+            WQ[k] = pf * PQ[k];
+            PB[k] = PA[k] + AB[k];
+            QD[k] = QC[k] + CD[k];
+        }
+        // h2p (S_m - qf S_m+1)
+        R e[LT];
+#pragma unroll
+        for (int m = 0; m < LT; m++) e[m] = h2p * gfma(-qf, S[m + 1], S[m]);
         if constexpr (L == 1) {
             if constexpr (LC == 0) {
 #pragma unroll
@@ -144,96 +145,126 @@ __device__ __forceinline__ void low_prim(R (&v)[low_nsum(LA, LB, LC, LD)], const
                 for (int k = 0; k < 3; k++)
 #pragma unroll
                     for (int i = 0; i < 3; i++) {
-                        R t = gfma(QC[k], P[0][i], v[i + 3 * k]);
+                        R t = WQ[k] * P[1][i];
                         if (i == k) t = gfma(hpq, S[1], t);
-                        v[i + 3 * k] = gfma(WQ[k], P[1][i], t);
+                        v[i + 3 * k] += gfma(QC[k], P[0][i], t);
                     }
             }
+        } else if constexpr (LA == 1) {
+            // (pp_j|ss)^m of one j at a time
+            constexpr int M = LC + 1;
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                R PP[M][3];
+#pragma unroll
+                for (int m = 0; m < M; m++)
+#pragma unroll
+                    for (int i = 0; i < 3; i++) {
+                        R t = WP[j] * P[m + 1][i];
+                        if (i == j) t += e[m];
+                        PP[m][i] = gfma(PB[j], P[m][i], t);
+                    }
+                if constexpr (LC == 0) {
+#pragma unroll
+                    for (int i = 0; i < 3; i++) v[i + 3 * j] += PP[0][i];
+                } else {
+                    const R sp = gfma(PB[j], S[1], WP[j] * S[2]);   // (s p_j|ss)^1
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+#pragma unroll
+                        for (int i = 0; i < 3; i++) {
+                            const int o = i + 3 * j + 9 * c;
+                            R t = WQ[c] * PP[1][i];
+                            if (i == c) t = gfma(hpq, sp, t);
+                            if (j == c) t = gfma(hpq, P[1][i], t);
+                            v[o] += gfma(QC[c], PP[0][i], t);
+                        }
+                }
+            }
         } else {
+            // (ds|ss)^m
             R D[LT - 1][6];
 #pragma unroll
-            for (int m = 0; m < LT - 1; m++) {
-                const R e = h2p * gfma(-qf, S[m + 1], S[m]);
+            for (int m = 0; m < LT - 1; m++)
 #pragma unroll
                 for (int i = 0; i < 3; i++)
 #pragma unroll
                     for (int j = i; j < 3; j++) {
                         R t = WP[j] * P[m + 1][i];
-                        if (i == j) t += e;
+                        if (i == j) t += e[m];
                         D[m][d_of(i, j)] = gfma(PA[j], P[m][i], t);
                     }
-            }
-            if constexpr (L >= 3) {
-                // (fs|ss)^m, each component from the (ds|ss) one that needs
-                // no delta term where there is such a one
-                R F[LT - 2][10];
+            if constexpr (LB > 0) {
+                // (dp_k|ss)^m of one k at a time
+                constexpr int M = LT - 2;
 #pragma unroll
-                for (int m = 0; m < LT - 2; m++) {
+                for (int k = 0; k < 3; k++) {
+                    R DP[M][6];
 #pragma unroll
-                    for (int i = 0; i < 3; i++)
+                    for (int m = 0; m < M; m++) {
+                        R pe[3];
 #pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            R t = WP[k] * D[m + 1][d_of(i, i)];
-                            if (i == k) t = gfma((R)2 * h2p, gfma(-qf, P[m + 1][k], P[m][k]), t);
-                            F[m][f_of(i, i, k)] = gfma(PA[k], D[m][d_of(i, i)], t);
-                        }
-                    F[m][4] = gfma(PA[2], D[m][1], WP[2] * D[m + 1][1]);   // xyz
-                }
-                if constexpr (L == 4) {
-                    // (gs|ss): xxxx.. from xxx, the others with as few delta terms as possible
-#pragma unroll
-                    for (int i = 0; i < 3; i++)
-#pragma unroll
-                        for (int k = 0; k < 3; k++) {
-                            const int f = f_of(i, i, i);
-                            R t = gfma(PA[k], F[0][f], v[g_of(i, i, i, k)]);
-                            if (i == k) t = gfma((R)3 * h2p, gfma(-qf, D[1][d_of(i, i)], D[0][d_of(i, i)]), t);
-                            v[g_of(i, i, i, k)] = gfma(WP[k], F[1][f], t);
-                        }
-#pragma unroll
-                    for (int i = 0; i < 3; i++) {
-                        const int j = (i + 1) % 3, k = (i + 2) % 3;
-                        // iijj from iij, iijk from iij
-                        const int f = f_of(i, i, j);
-                        R t = gfma(PA[j], F[0][f], v[g_of(i, i, j, j)]);
-                        t = gfma(h2p, gfma(-qf, D[1][d_of(i, i)], D[0][d_of(i, i)]), t);
-                        v[g_of(i, i, j, j)] = gfma(WP[j], F[1][f], t);
-                        v[g_of(i, i, j, k)] = gfma(WP[k], F[1][f], gfma(PA[k], F[0][f], v[g_of(i, i, j, k)]));
-                    }
-#pragma unroll
-                    for (int f = 0; f < 10; f++) v[15 + f] += F[0][f];
-#pragma unroll
-                    for (int d = 0; d < 6; d++) v[25 + d] += D[0][d];
-                } else if constexpr (LC == 0) {
-#pragma unroll
-                    for (int f = 0; f < 10; f++) v[f] += F[0][f];
-#pragma unroll
-                    for (int d = 0; d < 6; d++) v[10 + d] += D[0][d];
-                } else {
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
+                        for (int i = 0; i < 3; i++) pe[i] = h2p * gfma(-qf, P[m + 1][i], P[m][i]);
 #pragma unroll
                         for (int i = 0; i < 3; i++)
 #pragma unroll
                             for (int j = i; j < 3; j++) {
-                                R t = gfma(QC[c], D[0][d_of(i, j)], v[30 + d_of(i, j) + 6 * c]);
-                                if (i == c) t = gfma(hpq, P[1][j], t);
-                                if (j == c) t = gfma(hpq, P[1][i], t);
-                                v[30 + d_of(i, j) + 6 * c] = gfma(WQ[c], D[1][d_of(i, j)], t);
-#pragma unroll
-                                for (int k = j; k < 3; k++) {
-                                    const int f = f_of(i, j, k);
-                                    R u = gfma(QC[c], F[0][f], v[f + 10 * c]);
-                                    if (i == c) u = gfma(hpq, D[1][d_of(j, k)], u);
-                                    if (j == c) u = gfma(hpq, D[1][d_of(i, k)], u);
-                                    if (k == c) u = gfma(hpq, D[1][d_of(i, j)], u);
-                                    v[f + 10 * c] = gfma(WQ[c], F[1][f], u);
-                                }
+                                R t = WP[k] * D[m + 1][d_of(i, j)];
+                                if (i == k) t += pe[j];
+                                if (j == k) t += pe[i];
+                                DP[m][d_of(i, j)] = gfma(PB[k], D[m][d_of(i, j)], t);
                             }
+                    }
+                    if constexpr (LT == 3) {
+#pragma unroll
+                        for (int d = 0; d < 6; d++) v[d + 6 * k] += DP[0][d];
+                    } else {
+                        // (p_i p_k|ss)^m, from which the terms of a lowered d component follow
+                        R PP[2][3];
+#pragma unroll
+                        for (int m = 0; m < 2; m++)
+#pragma unroll
+                            for (int i = 0; i < 3; i++) {
+                                R t = WP[k] * P[m + 1][i];
+                                if (i == k) t += e[m];
+                                PP[m][i] = gfma(PB[k], P[m][i], t);
+                            }
+                        if constexpr (LC == 1) {
+#pragma unroll
+                            for (int c = 0; c < 3; c++)
+#pragma unroll
+                                for (int i = 0; i < 3; i++)
+#pragma unroll
+                                    for (int j = i; j < 3; j++) {
+                                        const int d = d_of(i, j), o = d + 6 * k + 18 * c;
+                                        R t = WQ[c] * DP[1][d];
+                                        if (k == c) t = gfma(hpq, D[1][d], t);
+                                        if (i == c) t = gfma(hpq, PP[1][j], t);
+                                        if (j == c) t = gfma(hpq, PP[1][i], t);
+                                        v[o] += gfma(QC[c], DP[0][d], t);
+                                    }
+                        } else {
+                            R pe[3];
+#pragma unroll
+                            for (int i = 0; i < 3; i++) pe[i] = h2p * gfma(-qf, PP[1][i], PP[0][i]);
+#pragma unroll
+                            for (int l = k; l < 3; l++)
+#pragma unroll
+                                for (int i = 0; i < 3; i++)
+#pragma unroll
+                                    for (int j = i; j < 3; j++) {
+                                        const int d = d_of(i, j), o = d + 6 * d_of(k, l);
+                                        R t = gfma(PB[l], DP[0][d], v[o]);
+                                        if (k == l) t = gfma(h2p, gfma(-qf, D[1][d], D[0][d]), t);
+                                        if (i == l) t += pe[j];
+                                        if (j == l) t += pe[i];
+                                        v[o] = gfma(WP[l], DP[1][d], t);
+                                    }
+                        }
                     }
                 }
             } else if constexpr (LC + LD == 2) {
-                // (ds|p_k s)^m, then (ds|d_kl s) with l >= k
+                // (ds|p_k s)^m, then (ds|d_kl s) with l >= k or (ds|p_k p_l)
 #pragma unroll
                 for (int k = 0; k < 3; k++) {
                     R DP[2][6], PP[3];
@@ -255,100 +286,37 @@ __device__ __forceinline__ void low_prim(R (&v)[low_nsum(LA, LB, LC, LD)], const
                         PP[i] = gfma(QC[k], P[1][i], t);
                     }
 #pragma unroll
-                    for (int l = k; l < 3; l++)
+                    for (int l = LD == 1 ? 0 : k; l < 3; l++)
 #pragma unroll
                         for (int i = 0; i < 3; i++)
 #pragma unroll
                             for (int j = i; j < 3; j++) {
-                                const int d = d_of(i, j), o = d + 6 * d_of(k, l);
-                                R t = gfma(QC[l], DP[0][d], v[o]);
+                                const int d = d_of(i, j), o = d + 6 * (LD == 1 ? k + 3 * l : d_of(k, l));
+                                R t = LD == 1 ? gfma(QD[l], DP[0][d], v[o]) : WQ[l] * DP[1][d];
                                 if (k == l) t = gfma(h2q, gfma(-pf, D[1][d], D[0][d]), t);
                                 if (i == l) t = gfma(hpq, PP[j], t);
                                 if (j == l) t = gfma(hpq, PP[i], t);
-                                v[o] = gfma(WQ[l], DP[1][d], t);
+                                if constexpr (LD == 1) v[o] = gfma(WQ[l], DP[1][d], t);
+                                else v[o] += gfma(QC[l], DP[0][d], t);
                             }
-                    if constexpr (LD == 1) {
-#pragma unroll
-                        for (int d = 0; d < 6; d++) v[36 + d + 6 * k] += DP[0][d];
-                    }
                 }
             } else if constexpr (LC == 0) {
 #pragma unroll
                 for (int d = 0; d < 6; d++) v[d] += D[0][d];
-                if constexpr (LB == 1) {
-#pragma unroll
-                    for (int i = 0; i < 3; i++) v[6 + i] += P[0][i];
-                }
             } else {
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
+                for (int k = 0; k < 3; k++)
 #pragma unroll
                     for (int i = 0; i < 3; i++)
 #pragma unroll
                         for (int j = i; j < 3; j++) {
                             const int d = d_of(i, j);
-                            R t = gfma(QC[k], D[0][d], v[d + 6 * k]);
+                            R t = WQ[k] * D[1][d];
                             if (i == k) t = gfma(hpq, P[1][j], t);
                             if (j == k) t = gfma(hpq, P[1][i], t);
-                            v[d + 6 * k] = gfma(WQ[k], D[1][d], t);
+                            v[d + 6 * k] += gfma(QC[k], D[0][d], t);
                         }
-                    if constexpr (LB == 1) {
-#pragma unroll
-                        for (int i = 0; i < 3; i++) {
-                            R t = gfma(QC[k], P[0][i], v[18 + i + 3 * k]);
-                            if (i == k) t = gfma(hpq, S[1], t);
-                            v[18 + i + 3 * k] = gfma(WQ[k], P[1][i], t);
-                        }
-                    }
-                }
             }
         }
-    }
-}
-
-// the quartet's integrals from the contracted sums:
-// acc[ia + NA*(ib + NB*(ic + NC*id))]
-template <int LA, int LB, int LC, int LD, typename R>
-__device__ __forceinline__ void low_finish(const R (&v)[low_nsum(LA, LB, LC, LD)], const R (&AB)[3], const R (&CD)[3],
-                                           R (&acc)[ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD)])
-{
-    constexpr int NA = ncart(LA);
-    if constexpr (LD == 1) {
-#pragma unroll
-        for (int id = 0; id < 3; id++)
-#pragma unroll
-            for (int ic = 0; ic < 3; ic++)
-#pragma unroll
-                for (int ia = 0; ia < NA; ia++)
-                    acc[ia + NA * (ic + 3 * id)] = gfma(CD[id], v[NA * 6 + ia + NA * ic], v[ia + NA * d_of(ic, id)]);
-    } else if constexpr (LB == 0) {
-#pragma unroll
-        for (int k = 0; k < NA * ncart(LC); k++) acc[k] = v[k];
-    } else if constexpr (LB == 1) {
-        constexpr int NU = ncart(LA + 1) * ncart(LC);
-#pragma unroll
-        for (int k = 0; k < ncart(LC); k++)
-#pragma unroll
-            for (int ib = 0; ib < 3; ib++)
-#pragma unroll
-                for (int ia = 0; ia < NA; ia++) {
-                    // component a + 1_b (ncart(LA + 1) of them)
-                    const int up = cart_of(cart_y(LA, ia) + (ib == 1), cart_z(LA, ia) + (ib == 2));
-                    acc[ia + NA * (ib + 3 * k)] = gfma(AB[ib], v[NU + ia + NA * k], v[up + ncart(LA + 1) * k]);
-                }
-    } else {
-        // (d d_jk| = (d+1_k p_j| + AB_k (d p_j|, (x p_j| = (x+1_j| + AB_j (x|
-#pragma unroll
-        for (int j = 0; j < 3; j++)
-#pragma unroll
-            for (int k = j; k < 3; k++)
-#pragma unroll
-                for (int ia = 0; ia < 6; ia++) {
-                    const int y = cart_y(2, ia), z = cart_z(2, ia);
-                    const R fj = v[15 + cart_of(y + (j == 1), z + (j == 2))], fk = v[15 + cart_of(y + (k == 1), z + (k == 2))];
-                    const R gjk = v[cart_of(y + (j == 1) + (k == 1), z + (j == 2) + (k == 2))];
-                    const R up = gfma(AB[j], fk, gjk), low = gfma(AB[j], v[25 + ia], fj);
-                    acc[ia + 6 * d_of(j, k)] = gfma(AB[k], low, up);
-                }
     }
 }

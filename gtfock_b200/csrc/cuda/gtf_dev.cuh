@@ -413,7 +413,6 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC), ND = ncart(LD);
     static_assert(!LOW || (low_class(LA, LB, LC, LD) && N == NC * ND), "whole quartets of the low classes");
-    R low[LOW ? low_nsum(LA, LB, LC, LD) : 1] = {};
     const R ABx = (R)pb.ABx, ABy = (R)pb.ABy, ABz = (R)pb.ABz;
     const R CDx = (R)pk.ABx, CDy = (R)pk.ABy, CDz = (R)pk.ABz;
     const int kstep = split & 0xff, bstep = (split >> 8) & 0xff, ik0 = (split >> 16) & 0xff, ib0 = split >> 24;
@@ -441,7 +440,8 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
 #pragma unroll
                 for (int m = 0; m <= LA + LB + LC + LD; m++) S[m] *= pref;
                 const R PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
-                low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (R)0.5 * ipq);
+                const R AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
+                low_prim<LA, LB, LC, LD>(acc, S, PA, AB, QC, CD, PQ, qf, pf, h2p, h2q, (R)0.5 * ipq);
                 continue;
             }
             const RysArg<NR, SPAD, R> rys(T, rtab);
@@ -491,10 +491,6 @@ __device__ __forceinline__ void eri_accumulate_cd(const PPB &bra, const PairRec 
         // not one bra primitive: both lists are in descending |K|
         if (SKIP && ib == ib0) break;
     }
-    if constexpr (LOW) {
-        const R AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
-        low_finish<LA, LB, LC, LD>(low, AB, CD, acc);
-    }
     (void)ND;
 }
 
@@ -509,7 +505,6 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
     constexpr int NR = (LA + LB + LC + LD) / 2 + 1;
     constexpr int NI = LA + LB + 1, NK = LC + LD + 1;
     constexpr int NA = ncart(LA), NB = ncart(LB), NC = ncart(LC);
-    float low[LOW ? low_nsum(LA, LB, LC, LD) : 1] = {};
     const float ABx = (float)pb.ABx, ABy = (float)pb.ABy, ABz = (float)pb.ABz;
     const float CDx = (float)pk.ABx, CDy = (float)pk.ABy, CDz = (float)pk.ABz;
     const float ACx = (float)(pb.Ax - pk.Ax), ACy = (float)(pb.Ay - pk.Ay), ACz = (float)(pb.Az - pk.Az);
@@ -539,7 +534,8 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
 #pragma unroll
                 for (int m = 0; m <= LA + LB + LC + LD; m++) S[m] *= pref;
                 const float PA[3] = {PAx, PAy, PAz}, QC[3] = {QCx, QCy, QCz}, PQ[3] = {PQx, PQy, PQz};
-                low_prim<LA, LB, LC, LD>(low, S, PA, QC, PQ, qf, pf, h2p, h2q, (float)0.5 * ipq);
+                const float AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
+                low_prim<LA, LB, LC, LD>(acc, S, PA, AB, QC, CD, PQ, qf, pf, h2p, h2q, (float)0.5 * ipq);
                 continue;
             }
             const RysArg<NR, SPAD, float> rys(T, rtab);
@@ -587,10 +583,6 @@ __device__ __forceinline__ void eri_accumulate_cd32(const PPRec32 &src, const Pa
         }
         // not one bra primitive: both lists are in descending |K|
         if (SKIP && ib == ib0) break;
-    }
-    if constexpr (LOW) {
-        const float AB[3] = {ABx, ABy, ABz}, CD[3] = {CDx, CDy, CDz};
-        low_finish<LA, LB, LC, LD>(low, AB, CD, acc);
     }
 }
 
