@@ -144,6 +144,7 @@ def load():
     _sig(L, "gtf_device_trim", [ctypes.c_size_t])
     _sig(L, "gtf_get_device", [_ip])
     _sig(L, "gtf_debug_fail_alloc", [_i], None)
+    _sig(L, "gtf_debug_fail_launch", [_i], None)
     _sig(L, "gtf_debug_live_allocs", [], ctypes.c_longlong)
     _sig(L, "gtf_pfock_compute_noalloc", [_vp, _vp, _vp])
     _sig(L, "gtf_shard_split", [_dp, ctypes.c_longlong, _i, _i, ctypes.POINTER(ctypes.c_longlong),

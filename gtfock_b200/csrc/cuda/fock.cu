@@ -111,95 +111,6 @@ struct ClassPairTask {
     long long *d_unit_prefix32;  // [nbra + 1], FP32 launch
 };
 
-// Side streams for the launches of one build, which are independent of one
-// another: fork() lets the first n - 1 of them start where fs.s[0] stands,
-// join() lets fs.s[0] go on once they are through.  The sets come from a
-// process-wide pool (creating one takes 0.3 ms) and return to it with the
-// engine or batch that took them, at most GTF_SIDE_SETS waiting there; a set
-// that returns has been waited for.
-#define GTF_SIDE_SETS 16
-struct SideStreams {
-    int dev;
-    cudaStream_t s[GTF_FOCK_STREAMS - 1];
-    cudaEvent_t ev_fork, ev_join[GTF_FOCK_STREAMS - 1];
-};
-static std::mutex g_side_mu;
-static std::vector<SideStreams *> g_side;
-
-static void side_destroy(SideStreams *p)
-{
-    for (int k = 0; k < GTF_FOCK_STREAMS - 1; k++) {
-        if (p->ev_join[k]) cudaEventDestroy(p->ev_join[k]);
-        if (p->s[k]) cudaStreamDestroy(p->s[k]);
-    }
-    if (p->ev_fork) cudaEventDestroy(p->ev_fork);
-    delete p;
-}
-
-struct ForkJoin {
-    SideStreams *p;
-    cudaError_t fork(FockStreams &fs, int n)
-    {
-        cudaError_t e = p ? cudaSuccess : take();
-        if (e == cudaSuccess) e = cudaEventRecord(p->ev_fork, fs.s[0]);
-        fs.n = n < 1 ? 1 : n > GTF_FOCK_STREAMS ? GTF_FOCK_STREAMS : n;
-        for (int k = 1; k < fs.n && e == cudaSuccess; k++) {
-            fs.s[k] = p->s[k - 1];
-            e = cudaStreamWaitEvent(fs.s[k], p->ev_fork, 0);
-        }
-        return e;
-    }
-    cudaError_t join(FockStreams &fs)
-    {
-        cudaError_t e = cudaSuccess;
-        for (int k = 1; k < fs.n && e == cudaSuccess; k++) {
-            e = cudaEventRecord(p->ev_join[k - 1], fs.s[k]);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(fs.s[0], p->ev_join[k - 1], 0);
-        }
-        return e;
-    }
-    cudaError_t take()
-    {
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e != cudaSuccess) return e;
-        {
-            std::lock_guard<std::mutex> lk(g_side_mu);
-            for (size_t k = 0; k < g_side.size(); k++)
-                if (g_side[k]->dev == dev) {
-                    p = g_side[k];
-                    g_side.erase(g_side.begin() + k);
-                    return cudaSuccess;
-                }
-        }
-        SideStreams *q = new SideStreams();
-        q->dev = dev;
-        e = cudaEventCreateWithFlags(&q->ev_fork, cudaEventDisableTiming);
-        for (int k = 0; k < GTF_FOCK_STREAMS - 1 && e == cudaSuccess; k++) {
-            e = cudaStreamCreateWithFlags(&q->s[k], cudaStreamNonBlocking);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&q->ev_join[k], cudaEventDisableTiming);
-        }
-        if (e == cudaSuccess) p = q;
-        else side_destroy(q);
-        return e;
-    }
-    void give_back()
-    {
-        if (!p) return;
-        // a build that failed between fork and join left work unjoined
-        for (cudaStream_t q : p->s) cudaStreamSynchronize(q);
-        {
-            std::lock_guard<std::mutex> lk(g_side_mu);
-            if (g_side.size() < GTF_SIDE_SETS) {
-                g_side.push_back(p);
-                p = nullptr;
-            }
-        }
-        if (p) side_destroy(p);
-        p = nullptr;
-    }
-};
-
 struct gtf_fock_dev {
     int dev;
     int nsm;
@@ -1053,8 +964,14 @@ typedef int (*fock_group_launch_t)(int la, int lb, int lc, int ld, const FockGri
 extern fock_group_launch_t gtf_fock_groups[];
 extern const int gtf_fock_ngroups;
 
+// Test hook: the n-th class launch from now on fails as a refused kernel
+// launch would (0: off).
+static std::atomic<int> g_fail_launch{0};
+extern "C" void gtf_debug_fail_launch(int n) { g_fail_launch.store(n); }
+
 static int launch_fock(int X, int Y, const FockGrid &fg, FockStreams &st)
 {
+    if (g_fail_launch.load(std::memory_order_relaxed) > 0 && g_fail_launch.fetch_sub(1) == 1) return -1;
     for (int g = 0; g < gtf_fock_ngroups; g++) {
         int r = gtf_fock_groups[g](k_cls_la[X], k_cls_lb[X], k_cls_la[Y], k_cls_lb[Y], fg, st);
         if (r != GTF_NOT_IN_GROUP) return r;  // launches, or -1 on error
@@ -1819,6 +1736,7 @@ extern "C" void gtf_fock_destroy(gtf_fock_dev_t *f)
 {
     if (!f) return;
     cudaStreamSynchronize(f->stream);
+    f->side.give_back();   // before the frees: it waits for the side streams
     cudaStream_t st = f->stream;
     void *ptrs[] = {f->d_sh_L, f->d_sh_nprim, f->d_sh_pstart, f->d_f_start, f->d_fc_start, f->d_sph2shell,
                     f->d_cart2shell, f->d_Z, f->d_sh_xyz, f->d_alpha, f->d_coef, f->d_atom_xyz, f->d_sq,
@@ -1847,7 +1765,6 @@ extern "C" void gtf_fock_destroy(gtf_fock_dev_t *f)
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : f->ev_cls)
         if (e) cudaEventDestroy(e);
-    f->side.give_back();
     if (f->stream) cudaStreamDestroy(f->stream);
     delete f;
 }
@@ -2191,6 +2108,7 @@ static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *
                           int konly = 0, bool dyn = false, bool timed = false, bool may_create = true)
 {
     FockStreams fs(f->stream);
+    ForkScope scope(f->side, fs);
     long long units = 0;
     int classes = 0;
     for (const ClassPairTask &t : f->tasks) {
@@ -2923,6 +2841,7 @@ extern "C" void gtf_fock_batch_destroy(gtf_fock_batch_t *b)
 {
     if (!b) return;
     cudaStreamSynchronize(b->st);
+    b->side.give_back();   // before the frees: it waits for the side streams
     cudaStream_t st = b->st;
     void *ptrs[] = {b->d_xf, b->d_counters, b->d_delta, b->d_full, b->d_ut, b->d_pdesc, b->d_ptot};
     for (void *p : ptrs) gtf_dfree(p, st);
@@ -2932,7 +2851,6 @@ extern "C" void gtf_fock_batch_destroy(gtf_fock_batch_t *b)
             gtf_dfree(b->d_desc[c][p], st);
             gtf_dfree(b->d_prefix[c][p], st);
         }
-    b->side.give_back();
     delete b;
 }
 
@@ -3194,6 +3112,7 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned long long) * (size_t)b->ncounter_blocks * GTF_MAX_SLICES,
                        st));
     FockStreams fs(st);
+    ForkScope scope(b->side, fs);
     long long units = 0;
     for (int c = 0; c < NCLSPAIR; c++)
         for (int p = 0; p < 2; p++) {

@@ -9,6 +9,7 @@
 
 #include "gtf_cuda.h"
 #include "gtf_dev.cuh"
+#include "side_streams.cuh"
 
 #define FOCK_THREADS 128
 
@@ -345,22 +346,6 @@ __global__ void __launch_bounds__(fock_max_threads(LA, LB, LC, LD, sizeof(R) == 
 // the counter, were as good for (H2O)64 but left C54H18's blocks unbalanced:
 // 190 ms against 182.)  Below, single units balance better.
 #define GTF_CHUNK_ROUNDS 16
-
-// Streams the launches of a build are dealt out to in turn (n == 1: all in
-// order on one stream).
-#define GTF_FOCK_STREAMS 8
-struct FockStreams {
-    cudaStream_t s[GTF_FOCK_STREAMS];
-    int n, next;
-    cudaStream_t last;   // stream of the latest launch
-    explicit FockStreams(cudaStream_t st) : n(1), next(0), last(st) { s[0] = st; }
-    cudaStream_t take()
-    {
-        last = s[next];
-        next = next + 1 < n ? next + 1 : 0;
-        return last;
-    }
-};
 
 // Number of slice launches of a class pair; g.counter points at that many
 // zeroed counters.

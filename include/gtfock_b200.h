@@ -288,6 +288,9 @@ void gtf_debug_fail_alloc(int n);
 /* Device allocations made through that hook's allocator (engine set-up and
  * engine buffers) that have not been freed yet. */
 long long gtf_debug_live_allocs(void);
+/* Test hook: the n-th launch of a class pair's kernels from now on is refused
+ * on the host, as a failed kernel launch would be (n <= 0 disarms). */
+void gtf_debug_fail_launch(int n);
 
 /* Number of this library's own kernel launches so far (all threads). */
 unsigned long long gtf_launch_count(void);

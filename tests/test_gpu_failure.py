@@ -5,6 +5,9 @@
   cudaMalloc would) returns PFOCK_STATUS_ALLOC_FAILED
   (pfock/pfock.h:188-202), leaves no device allocation behind, and the next
   engine works: every allocation point of the set-up is tried.
+* A refused launch in the middle of a build that runs over several streams
+  (gtf_debug_fail_launch): the build fails, the next one is right, and an
+  engine destroyed straight after the failure frees nothing still in use.
 * A request withdrawn from the batched engine between steps frees its slot;
   the other jobs finish exactly as they do without it."""
 import ctypes
@@ -54,6 +57,31 @@ def test_create_alloc_failure_releases_everything(tmp_path):
     # the library still works after the failures
     pf = gb.PFock(b, tolscr=float(g["tol"]))
     assert np.abs(pf.compute_fock(g["D"]) - g["F"]).max() < 1e-10
+    pf.close()
+
+
+def test_refused_launch_leaves_nothing_behind(tmp_path):
+    L = gb.load()
+    g = load_golden("c4h10_ccpvdz")
+    gbs, xyz = golden_xyz(g, tmp_path)
+    b = gb.BasisSet(gbs, xyz)
+    pf = gb.PFock(b, tolscr=float(g["tol"]))
+    for n in (1, 2, 9, 20):          # of 21 class pairs
+        L.gtf_debug_fail_launch(n)
+        with pytest.raises(RuntimeError):
+            pf.compute_fock(g["D"])
+        L.gtf_debug_fail_launch(0)
+        assert np.abs(pf.compute_fock(g["D"]) - g["F"]).max() < 1e-10
+        # destroyed straight after the failure; its memory goes to the next engine
+        other = gb.PFock(b, tolscr=float(g["tol"]))
+        L.gtf_debug_fail_launch(n)
+        with pytest.raises(RuntimeError):
+            other.compute_fock(g["D"])
+        L.gtf_debug_fail_launch(0)
+        other.close()
+        third = gb.PFock(b, tolscr=float(g["tol"]))
+        assert np.abs(third.compute_fock(g["D"]) - g["F"]).max() < 1e-10
+        third.close()
     pf.close()
 
 
