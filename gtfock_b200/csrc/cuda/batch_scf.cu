@@ -980,7 +980,8 @@ static int rebuild_fock_batch(gtf_batch *b, const std::vector<int> &run)
     b->fock_exec = nullptr;
     b->fock_launches = 0;
     cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    if (gtf_fock_batch_hold_streams(b->fb, 1) == GTF_OK &&
+        cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
         const int nl = gtf_fock_batch_compute(b->fb);
         const cudaError_t ce = cudaStreamEndCapture(b->st, &graph);
         if (nl >= 0 && ce == cudaSuccess && graph &&
@@ -993,6 +994,7 @@ static int rebuild_fock_batch(gtf_batch *b, const std::vector<int> &run)
         if (graph) cudaGraphDestroy(graph);
         cudaGetLastError();
     }
+    gtf_fock_batch_hold_streams(b->fb, 0);
     // tile shape of the dense products: tuned for this size, else 64 x 64, or
     // 32 x 32 where those tiles would leave SMs idle
     long long tiles = 0;

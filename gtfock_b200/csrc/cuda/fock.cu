@@ -148,7 +148,6 @@ struct gtf_fock_dev {
     // timing
     cudaEvent_t ev0, ev1, ev2, ev3;
     cudaEvent_t ev_cls[2 * NCLSPAIR];   // start and end of each class pair's launches
-    ForkJoin side;
     double ms_total, ms_eri, ms_other;
     double ms_cls[NCLSPAIR];
     int prec;
@@ -1736,7 +1735,6 @@ extern "C" void gtf_fock_destroy(gtf_fock_dev_t *f)
 {
     if (!f) return;
     cudaStreamSynchronize(f->stream);
-    f->side.give_back();   // before the frees: it waits for the side streams
     cudaStream_t st = f->stream;
     void *ptrs[] = {f->d_sh_L, f->d_sh_nprim, f->d_sh_pstart, f->d_f_start, f->d_fc_start, f->d_sph2shell,
                     f->d_cart2shell, f->d_Z, f->d_sh_xyz, f->d_alpha, f->d_coef, f->d_atom_xyz, f->d_sq,
@@ -2102,13 +2100,13 @@ static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *F
 // times per class pair would no longer add up.
 #define GTF_OVERLAP_UNITS 2000000LL
 
-// All class pairs of one build; timed: events around each; may_create: the
-// side streams may be created.
+// All class pairs of one build; timed: events around each; may_create: side
+// streams may be created where none waits in the pool.
 static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *Fk, unsigned long long *counters,
                           int konly = 0, bool dyn = false, bool timed = false, bool may_create = true)
 {
     FockStreams fs(f->stream);
-    ForkScope scope(f->side, fs);
+    SideLease side;
     long long units = 0;
     int classes = 0;
     for (const ClassPairTask &t : f->tasks) {
@@ -2116,7 +2114,8 @@ static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *
         classes += t.nbra > 0 && t.nketcls > 0;
     }
     // 6 class pairs of s and p shells: few launches; with d shells 62
-    if (units <= GTF_OVERLAP_UNITS && (f->side.p || may_create)) CK(f->side.fork(fs, classes));
+    if (units <= GTF_OVERLAP_UNITS) CK(side.take(f->stream, may_create));
+    if (side.p) CK(side.fork(fs, classes));
     for (int c = 0; c < NCLSPAIR; c++) {
         if (f->tasks[c].nbra == 0 || f->tasks[c].nketcls == 0) continue;
         if (timed) CK(cudaEventRecord(f->ev_cls[2 * c], fs.s[fs.next]));
@@ -2126,7 +2125,7 @@ static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *
         gtf_note_launches(r);
         if (timed) CK(cudaEventRecord(f->ev_cls[2 * c + 1], fs.last));
     }
-    CK(f->side.join(fs));
+    CK(side.join());
     return GTF_OK;
 }
 
@@ -2799,7 +2798,7 @@ struct gtf_fock_batch {
     int npdesc;
     size_t maxnn;
     std::vector<const long long *> solo_tot[NCLSPAIR][2];
-    ForkJoin side;
+    SideLease held;   // side streams of a build under capture
 };
 
 // A molecule whose units in one launch reach this many (32 quartets each)
@@ -2841,7 +2840,6 @@ extern "C" void gtf_fock_batch_destroy(gtf_fock_batch_t *b)
 {
     if (!b) return;
     cudaStreamSynchronize(b->st);
-    b->side.give_back();   // before the frees: it waits for the side streams
     cudaStream_t st = b->st;
     void *ptrs[] = {b->d_xf, b->d_counters, b->d_delta, b->d_full, b->d_ut, b->d_pdesc, b->d_ptot};
     for (void *p : ptrs) gtf_dfree(p, st);
@@ -3078,6 +3076,25 @@ extern "C" int gtf_fock_batch_set_full(gtf_fock_batch_t *b, const int *full)
     return GTF_OK;
 }
 
+// few enough units for launches over several streams (GTF_OVERLAP_UNITS)
+static bool batch_overlaps(const gtf_fock_batch *b)
+{
+    long long units = 0;
+    for (int c = 0; c < NCLSPAIR; c++)
+        for (int p = 0; p < 2; p++) {
+            units += b->total[c][p];
+            for (long long n : b->solo_units[c][p]) units += n;
+        }
+    return units <= GTF_OVERLAP_UNITS;
+}
+
+extern "C" int gtf_fock_batch_hold_streams(gtf_fock_batch_t *b, int hold)
+{
+    if (!hold) b->held.release();
+    else if (batch_overlaps(b)) CK(b->held.take(b->st));
+    return GTF_OK;
+}
+
 extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
 {
     cudaStream_t st = b->st;
@@ -3112,14 +3129,10 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
     CK(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned long long) * (size_t)b->ncounter_blocks * GTF_MAX_SLICES,
                        st));
     FockStreams fs(st);
-    ForkScope scope(b->side, fs);
-    long long units = 0;
-    for (int c = 0; c < NCLSPAIR; c++)
-        for (int p = 0; p < 2; p++) {
-            units += b->total[c][p];
-            for (long long n : b->solo_units[c][p]) units += n;
-        }
-    if (units <= GTF_OVERLAP_UNITS) CK(b->side.fork(fs, GTF_FOCK_STREAMS));
+    SideLease own, &side = b->held.p ? b->held : own;
+    const ForkScope scope(side);
+    if (batch_overlaps(b)) CK(side.take(st));
+    if (side.p) CK(side.fork(fs, GTF_FOCK_STREAMS));
     for (int c = 0; c < NCLSPAIR; c++) {
         const ClassPairTask &t0 = b->eng[0]->tasks[c];
         for (int p = 0; p < 2; p++) {
@@ -3164,7 +3177,7 @@ extern "C" int gtf_fock_batch_compute(gtf_fock_batch_t *b)
             launches += r;
         }
     }
-    CK(b->side.join(fs));
+    CK(side.join());
     {
         dim3 g((b->maxn + 127) / 128, b->maxn < 1024 ? b->maxn : 1024, b->M);
         k_b_post<<<g, 128, 0, st>>>(b->d_xf);

@@ -96,6 +96,10 @@ int gtf_fock_eri_flops(gtf_fock_dev_t *f, double *flops);
  * own density buffer (gtf_fock_mat_dev(f, 0, 0)) and fills its own F/J/K. */
 typedef struct gtf_fock_batch gtf_fock_batch_t;
 int gtf_fock_batch_create(gtf_fock_dev_t *const *engines, int M, void *stream, gtf_fock_batch_t **out);
+/* Takes (hold != 0) and returns the side streams of the batch's builds: a
+ * build inside a stream capture runs over several streams only if they were
+ * taken before it, and they are kept until it ends. */
+int gtf_fock_batch_hold_streams(gtf_fock_batch_t *b, int hold);
 int gtf_fock_batch_compute(gtf_fock_batch_t *b);
 /* incremental batches: full[m] != 0 makes member m's next build a full one */
 int gtf_fock_batch_set_full(gtf_fock_batch_t *b, const int *full);

@@ -23,10 +23,10 @@ struct FockStreams {
     }
 };
 
-// fork() lets the first n - 1 side streams start where fs.s[0] stands, join()
-// lets fs.s[0] go on once they are through.  The sets come from a
-// process-wide pool (creating one takes 0.3 ms) and return to it with the
-// engine or batch that took them, at most GTF_SIDE_SETS waiting there.
+// A set of side streams.  Sets are leased for one build: they come from a
+// process-wide pool (creating one takes 0.3 ms), so there are as many as
+// builds that were ever under way at once, and at most GTF_SIDE_SETS wait in
+// the pool.
 #define GTF_SIDE_SETS 16
 struct SideStreams {
     int dev;
@@ -53,38 +53,31 @@ inline void side_destroy(SideStreams *p)
     delete p;
 }
 
-struct ForkJoin {
+// The lease of one build.  fork() lets the first n - 1 side streams start
+// where fs.s[0] stands, join() lets fs.s[0] go on once they are through.  The
+// end of the lease joins on every way out, a failed launch among them, so that
+// a retry's clears and the frees of a destroyed engine come after all that was
+// launched, and returns the set.  The set may still be busy then: what its
+// next user launches comes after that.
+struct SideLease {
     SideStreams *p;
-    cudaError_t fork(FockStreams &fs, int n)
+    FockStreams *fs;   // forked and not joined
+    SideLease() : p(nullptr), fs(nullptr) {}
+    SideLease(const SideLease &) = delete;
+    SideLease &operator=(const SideLease &) = delete;
+    ~SideLease() { release(); }
+    // Takes a set of the current device for a build on `st`: from the pool,
+    // or a new one if none waits there.  The lease stays empty without
+    // `create`, or when `st` is being captured: a set belongs to a capture
+    // until that ends, so whoever captures takes it before and keeps it.
+    cudaError_t take(cudaStream_t st, bool create = true)
     {
-        cudaError_t e = p ? cudaSuccess : take();
-        if (e == cudaSuccess) e = cudaEventRecord(p->ev_fork, fs.s[0]);
-        fs.n = n < 1 ? 1 : n > GTF_FOCK_STREAMS ? GTF_FOCK_STREAMS : n;
-        for (int k = 1; k < fs.n && e == cudaSuccess; k++) {
-            fs.s[k] = p->s[k - 1];
-            e = cudaStreamWaitEvent(fs.s[k], p->ev_fork, 0);
-        }
-        if (e != cudaSuccess) fs.n = 1;   // nothing was launched on the others
-        return e;
-    }
-    // whatever fails, fs.s[0] waits for every stream it can
-    cudaError_t join(FockStreams &fs)
-    {
-        cudaError_t first = cudaSuccess;
-        for (int k = 1; k < fs.n; k++) {
-            cudaError_t e = cudaEventRecord(p->ev_join[k - 1], fs.s[k]);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(fs.s[0], p->ev_join[k - 1], 0);
-            if (e != cudaSuccess) cudaStreamSynchronize(fs.s[k]);
-            if (first == cudaSuccess) first = e;
-        }
-        fs.n = 1;
-        fs.next = 0;
-        return first;
-    }
-    cudaError_t take()
-    {
+        if (p) return cudaSuccess;
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(st, &cap);
+        if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) return e;
         int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
+        e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
         {
             std::lock_guard<std::mutex> lk(side_pool().mu);
@@ -96,6 +89,7 @@ struct ForkJoin {
                     return cudaSuccess;
                 }
         }
+        if (!create) return cudaSuccess;
         SideStreams *q = new SideStreams();
         q->dev = dev;
         e = cudaEventCreateWithFlags(&q->ev_fork, cudaEventDisableTiming);
@@ -107,12 +101,40 @@ struct ForkJoin {
         else side_destroy(q);
         return e;
     }
-    // The builds that used the set have been joined: what is left on it is
-    // ordered before the work the owner's stream, and its next user's, has.
-    void give_back()
+    // needs a set
+    cudaError_t fork(FockStreams &f, int n)
     {
+        cudaError_t e = cudaEventRecord(p->ev_fork, f.s[0]);
+        f.n = n < 1 ? 1 : n > GTF_FOCK_STREAMS ? GTF_FOCK_STREAMS : n;
+        for (int k = 1; k < f.n && e == cudaSuccess; k++) {
+            f.s[k] = p->s[k - 1];
+            e = cudaStreamWaitEvent(f.s[k], p->ev_fork, 0);
+        }
+        if (e == cudaSuccess) fs = &f;
+        else f.n = 1;   // nothing was launched on the others
+        return e;
+    }
+    // whatever fails, fs.s[0] waits for every stream it can
+    cudaError_t join()
+    {
+        cudaError_t first = cudaSuccess;
+        for (int k = 1; fs && k < fs->n; k++) {
+            cudaError_t e = cudaEventRecord(p->ev_join[k - 1], fs->s[k]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(fs->s[0], p->ev_join[k - 1], 0);
+            if (e != cudaSuccess) cudaStreamSynchronize(fs->s[k]);
+            if (first == cudaSuccess) first = e;
+        }
+        if (fs) {
+            fs->n = 1;
+            fs->next = 0;
+        }
+        fs = nullptr;
+        return first;
+    }
+    void release()
+    {
+        join();
         if (!p) return;
-        for (cudaStream_t q : p->s) cudaStreamSynchronize(q);
         {
             std::lock_guard<std::mutex> lk(side_pool().mu);
             if (side_pool().idle.size() < GTF_SIDE_SETS) {
@@ -120,19 +142,14 @@ struct ForkJoin {
                 p = nullptr;
             }
         }
-        if (p) side_destroy(p);
+        if (p) side_destroy(p);   // a busy stream is destroyed when its work is done
         p = nullptr;
     }
 };
 
-// Joins the streams of a fork on every way out, a failed launch among them:
-// the caller's stream is then ordered behind all that was launched, so a
-// retry's clears and the frees of a destroyed engine come after it.
+// joins a lease that outlives the build
 struct ForkScope {
-    ForkJoin &fj;
-    FockStreams &fs;
-    ForkScope(ForkJoin &f, FockStreams &s) : fj(f), fs(s) {}
-    ~ForkScope() { fj.join(fs); }
-    ForkScope(const ForkScope &) = delete;
-    ForkScope &operator=(const ForkScope &) = delete;
+    SideLease &side;
+    explicit ForkScope(SideLease &l) : side(l) {}
+    ~ForkScope() { side.join(); }
 };

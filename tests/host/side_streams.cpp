@@ -21,17 +21,19 @@ static int launch(FockStreams &fs)
     return next_launch++;
 }
 
-// a build of n launches after `clear` on the main stream; fail: stops after that many
-static cudaError_t build(ForkJoin &side, cudaStream_t main, int n, int fail)
+// a build of n launches after what `main` holds; fail: stops after that many
+static cudaError_t build(cudaStream_t main, int n, int fail, SideLease *held = nullptr)
 {
     FockStreams fs(main);
-    ForkScope scope(side, fs);
-    if (side.fork(fs, n) != cudaSuccess) return cudaErrorUnknown;
+    SideLease own, &side = held ? *held : own;
+    const ForkScope scope(side);
+    if (side.take(main) != cudaSuccess) return cudaErrorUnknown;
+    if (side.p && side.fork(fs, n) != cudaSuccess) return cudaErrorUnknown;
     for (int k = 0; k < n; k++) {
         if (k == fail) return cudaErrorUnknown;
         launch(fs);
     }
-    return side.join(fs);
+    return side.join();
 }
 
 // every launch from `first` on
@@ -48,24 +50,57 @@ int main()
         FakeStream main_stream;
         const int first = next_launch;
         main_stream.behind.insert(next_launch++);   // the clears
-        ForkJoin side{nullptr};
-        const cudaError_t e = build(side, &main_stream, 12, fail);
+        const cudaError_t e = build(&main_stream, 12, fail);
         CHECK((e == cudaSuccess) == (fail < 0));
-        CHECK(behind_all(&main_stream, first));            // a retry, or a free, comes after every launch
-        side.give_back();
+        CHECK(behind_all(&main_stream, first));     // a retry, or a free, comes after every launch
     }
     // a record of the join fails: the host waits for that stream instead
     for (int rec = 1; rec <= 8; rec++) {
         FakeStream main_stream;
         const int first = next_launch;
-        ForkJoin side{nullptr};
         fake_fail_record = rec;
-        CHECK(build(side, &main_stream, 12, -1) != cudaSuccess);
+        CHECK(build(&main_stream, 12, -1) != cudaSuccess);
         fake_fail_record = 0;
         CHECK(behind_all(&main_stream, first));
-        side.give_back();
     }
-    CHECK(side_pool().idle.size() == 1);            // one set served every build
+    // leased for the build: one set served every one of them
+    CHECK(side_pool().idle.size() == 1);
     CHECK(fake_streams == GTF_FOCK_STREAMS - 1 && fake_events == GTF_FOCK_STREAMS);
+
+    // under capture: no set is taken or created inside; one taken before is used and kept
+    side_pool().idle.clear();
+    fake_streams = fake_events = 0;
+    FakeStream captured;
+    SideLease held;
+    CHECK(held.take(&captured) == cudaSuccess && held.p);
+    SideStreams *set = held.p;
+    const int made = fake_streams;
+    captured.capturing = true;
+    CHECK(build(&captured, 12, -1) == cudaSuccess && side_pool().idle.empty() && fake_streams == made);
+    const int first = next_launch;
+    CHECK(build(&captured, 12, 5, &held) != cudaSuccess);
+    CHECK(behind_all(&captured, first));
+    CHECK(build(&captured, 12, -1, &held) == cudaSuccess);
+    CHECK(behind_all(&captured, first));
+    CHECK(held.p == set && side_pool().idle.empty());
+    captured.capturing = false;
+    held.release();
+    CHECK(side_pool().idle.size() == 1);
+
+    // no set waits and none may be created
+    side_pool().idle.clear();
+    FakeStream plain;
+    SideLease none;
+    CHECK(none.take(&plain, false) == cudaSuccess && !none.p);
+
+    // at most GTF_SIDE_SETS wait in the pool
+    fake_streams = 0;
+    {
+        SideLease many[GTF_SIDE_SETS + 3];
+        for (SideLease &l : many) CHECK(l.take(&plain) == cudaSuccess);
+        CHECK(fake_streams == (GTF_SIDE_SETS + 3) * (GTF_FOCK_STREAMS - 1));
+    }
+    CHECK(side_pool().idle.size() == GTF_SIDE_SETS);
+    CHECK(fake_streams == GTF_SIDE_SETS * (GTF_FOCK_STREAMS - 1));
     return 0;
 }

@@ -6,8 +6,10 @@
 typedef int cudaError_t;
 enum { cudaSuccess = 0, cudaErrorUnknown = 999 };
 enum { cudaEventDisableTiming = 2, cudaStreamNonBlocking = 1 };
+enum cudaStreamCaptureStatus { cudaStreamCaptureStatusNone, cudaStreamCaptureStatusActive };
 struct FakeStream {
     std::set<int> behind;
+    bool capturing = false;
 };
 struct FakeEvent {
     std::set<int> at;
@@ -39,5 +41,10 @@ inline cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, int)
 inline cudaError_t cudaStreamSynchronize(cudaStream_t s)
 {
     fake_done.insert(s->behind.begin(), s->behind.end());
+    return cudaSuccess;
+}
+inline cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus *c)
+{
+    *c = s->capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
