@@ -150,6 +150,10 @@ struct gtf_fock_dev {
     cudaEvent_t ev_cls[2 * NCLSPAIR];   // start and end of each class pair's launches
     double ms_total, ms_eri, ms_other;
     double ms_cls[NCLSPAIR];
+    // a build whose launches overlapped: its class times are measured when
+    // asked for, from this density and list kind (cls_builds densities; 0: ms_cls is current)
+    int cls_overlap, cls_builds, cls_dyn;
+    const double *cls_D;
     int prec;
     double fp32_cutoff;
     size_t dev_bytes;
@@ -2100,10 +2104,12 @@ static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *F
 // times per class pair would no longer add up.
 #define GTF_OVERLAP_UNITS 2000000LL
 
-// All class pairs of one build; timed: events around each; may_create: side
-// streams may be created where none waits in the pool.
+// All class pairs of one build; timed: events around each, if they run one
+// after another (f->cls_overlap); may_create: side streams may be created
+// where none waits in the pool.
 static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *Fk, unsigned long long *counters,
-                          int konly = 0, bool dyn = false, bool timed = false, bool may_create = true)
+                          int konly = 0, bool dyn = false, bool timed = false, bool may_create = true,
+                          bool may_overlap = true)
 {
     FockStreams fs(f->stream);
     SideLease side;
@@ -2114,19 +2120,60 @@ static int launch_classes(gtf_fock_dev *f, const double *D, double *Fj, double *
         classes += t.nbra > 0 && t.nketcls > 0;
     }
     // 6 class pairs of s and p shells: few launches; with d shells 62
-    if (units <= GTF_OVERLAP_UNITS) CK(side.take(f->stream, may_create));
+    if (units <= GTF_OVERLAP_UNITS && may_overlap) CK(side.take(f->stream, may_create));
     if (side.p) CK(side.fork(fs, classes));
+    if (timed) f->cls_overlap = side.p != nullptr;
+    timed = timed && !side.p;
     for (int c = 0; c < NCLSPAIR; c++) {
         if (f->tasks[c].nbra == 0 || f->tasks[c].nketcls == 0) continue;
-        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c], fs.s[fs.next]));
-        fs.last = fs.s[fs.next];
+        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c], f->stream));
         const int r = launch_class(f, c, D, Fj, Fk, counters, fs, konly, dyn);
         if (r < 0) return GTF_ERR_CUDA;
         gtf_note_launches(r);
-        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c + 1], fs.last));
+        if (timed) CK(cudaEventRecord(f->ev_cls[2 * c + 1], f->stream));
     }
     CK(side.join());
     return GTF_OK;
+}
+
+// Class times of a build that has finished: added up over its densities.
+static int add_class_times(gtf_fock_dev *f, const double *D, bool dyn, bool first)
+{
+    if (first) {
+        memset(f->ms_cls, 0, sizeof(f->ms_cls));
+        f->cls_builds = 0;
+    }
+    if (f->cls_overlap) {
+        f->cls_builds++;
+        f->cls_D = D;
+        f->cls_dyn = dyn;
+        return GTF_OK;
+    }
+    for (int c = 0; c < NCLSPAIR; c++) {
+        if (f->tasks[c].nbra == 0 || f->tasks[c].nketcls == 0) continue;
+        float ms = 0.0f;
+        CK(cudaEventElapsedTime(&ms, f->ev_cls[2 * c], f->ev_cls[2 * c + 1]));
+        f->ms_cls[c] += ms;
+    }
+    return GTF_OK;
+}
+
+// The launches of an overlapped build once more, one class after another, for
+// their times; F, J and K stay as they are.
+static int measure_class_times(gtf_fock_dev *f)
+{
+    const int builds = f->cls_builds;
+    if (builds == 0) return GTF_OK;
+    const size_t nnc = (size_t)f->nbf_cart * f->nbf_cart;
+    CK(cudaMemsetAsync(f->d_Fj, 0, sizeof(double) * nnc, f->stream));
+    CK(cudaMemsetAsync(f->d_Fk, 0, sizeof(double) * nnc, f->stream));
+    CK(cudaMemsetAsync(f->d_counters, 0, sizeof(unsigned long long) * 2 * NCLSPAIR * GTF_MAX_SLICES, f->stream));
+    int r = launch_classes(f, f->cls_D, f->d_Fj, f->d_Fk, f->d_counters, 0, f->cls_dyn != 0, true, false, false);
+    if (r) return r;
+    CK(cudaStreamSynchronize(f->stream));
+    r = add_class_times(f, nullptr, false, true);
+    for (double &ms : f->ms_cls) ms *= builds;
+    return r;
 }
 
 // One incremental build of density 0 (see k_delta): the change of D since
@@ -2181,12 +2228,8 @@ static int fock_compute_incremental(gtf_fock_dev *f)
     float tot = 0.0f, eri = 0.0f;
     CK(cudaEventElapsedTime(&tot, f->ev0, f->ev3));
     CK(cudaEventElapsedTime(&eri, f->ev1, f->ev2));
-    for (int c = 0; c < NCLSPAIR; c++) {
-        float mc = 0.0f;
-        if (f->tasks[c].nbra > 0 && f->tasks[c].nketcls > 0)
-            CK(cudaEventElapsedTime(&mc, f->ev_cls[2 * c], f->ev_cls[2 * c + 1]));
-        f->ms_cls[c] = mc;
-    }
+    r = add_class_times(f, Dc, true, true);
+    if (r) return r;
     f->ms_total = tot;
     f->ms_eri = eri;
     f->ms_other = tot - eri;
@@ -2326,12 +2369,8 @@ extern "C" int gtf_fock_compute(gtf_fock_dev_t *f, int numdmat)
         float ms = 0.0f;
         CK(cudaEventElapsedTime(&ms, f->ev1, f->ev2));
         eri_ms_total += ms;
-        for (int c = 0; c < NCLSPAIR; c++) {
-            float mc = 0.0f;
-            if (f->tasks[c].nbra > 0 && f->tasks[c].nketcls > 0)
-                CK(cudaEventElapsedTime(&mc, f->ev_cls[2 * c], f->ev_cls[2 * c + 1]));
-            f->ms_cls[c] = (d == 0 ? 0.0 : f->ms_cls[c]) + mc;
-        }
+        r = add_class_times(f, Dc, false, d == 0);
+        if (r) return r;
     }
     float tot = 0.0f;
     CK(cudaEventElapsedTime(&tot, f->ev0, f->ev3));
@@ -2412,6 +2451,8 @@ extern "C" int gtf_fock_last_timing(gtf_fock_dev_t *f, double *ms_total, double 
 // per class pair of the last build: (X, Y) classes, ms, quartets, Rys-model FLOPs
 extern "C" int gtf_fock_class_stats(gtf_fock_dev_t *f, int *X, int *Y, double *ms, double *nquart)
 {
+    const int r = ms ? measure_class_times(f) : GTF_OK;
+    if (r) return r;   // negative
     for (int c = 0; c < NCLSPAIR; c++) {
         if (X) X[c] = f->tasks[c].X;
         if (Y) Y[c] = f->tasks[c].Y;

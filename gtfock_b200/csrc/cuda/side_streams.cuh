@@ -13,13 +13,12 @@
 struct FockStreams {
     cudaStream_t s[GTF_FOCK_STREAMS];
     int n, next;
-    cudaStream_t last;   // stream of the latest launch
-    explicit FockStreams(cudaStream_t st) : n(1), next(0), last(st) { s[0] = st; }
+    explicit FockStreams(cudaStream_t st) : n(1), next(0) { s[0] = st; }
     cudaStream_t take()
     {
-        last = s[next];
+        const cudaStream_t st = s[next];
         next = next + 1 < n ? next + 1 : 0;
-        return last;
+        return st;
     }
 };
 

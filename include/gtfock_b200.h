@@ -35,9 +35,10 @@ PFockStatus_t gtf_pfock_timing(PFock_t pfock, double *ms_total, double *ms_eri,
 
 /* Per angular-class-pair statistics of the last build (21 pairs for s/p/d
  * shells): bra / ket pair classes (ss=0 ps=1 pp=2 ds=3 dp=4 dd=5), CUDA-event
- * ms of each class kernel and its quartet count.  Small builds run their
- * launches over several streams: their times are spans that overlap.  Returns
- * the pair count. */
+ * ms of each class pair's kernels and its quartet count.  Small builds run their
+ * kernels side by side; their class times are measured by this call, which then
+ * launches the kernels of the last build again, one class pair after another
+ * (F, J and K stay as they are).  Returns the pair count, or a negative error. */
 int gtf_pfock_class_stats(PFock_t pfock, int *X, int *Y, double *ms, double *nquart);
 
 /* Per class pair (same order): Rys-model FLOPs of one build and the number of
