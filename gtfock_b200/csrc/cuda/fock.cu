@@ -987,7 +987,7 @@ static int launch_fock(int X, int Y, const FockGrid &fg, FockStreams &st)
 // ---------------------------------------------------------------------------
 // Process-wide table: (kind, class X, class Y, precision part, size bucket)
 // -> (a, b).  Kind 0 / 1: a Fock launch of a single engine / of a batch,
-// a = persistent blocks per SM, b = units of 32 quartets a warp claims at
+// a = persistent blocks per SM, b = units of 32 lanes a warp claims at
 // once; kind 2: the batched dense products, a = tile shape.  The size bucket
 // is floor(log2) of the launch's units (or of the products' n^3 sum).  The
 // tuners time candidate shapes on the live engine and record the fastest;
@@ -1070,8 +1070,11 @@ static void device_name(char *out, size_t len)
         if (*c == ' ') *c = '_';
 }
 
-// Text file: "gtfock_b200-tune 1 <device>" then one entry per line
-// "kind X Y part bucket a b ms".
+// Text file: "gtfock_b200-tune <version> <device>" then one entry per line
+// "kind X Y part bucket a b ms".  The version names the launch shapes that the
+// Fock entries were measured on: 1, units of 32 quartets on small blocks; 2,
+// units of 32 lanes, one large block per SM at the occupancy limit.
+#define GTF_TUNE_VERSION 2
 extern "C" int gtf_tune_save(const char *path)
 {
     char dev[256];
@@ -1079,7 +1082,7 @@ extern "C" int gtf_tune_save(const char *path)
     FILE *fp = fopen(path, "w");
     if (!fp) return GTF_ERR_IO;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    fprintf(fp, "gtfock_b200-tune 1 %s\n", dev);
+    fprintf(fp, "gtfock_b200-tune %d %s\n", GTF_TUNE_VERSION, dev);
     for (const auto &kv : g_tune)
         fprintf(fp, "%d %d %d %d %d %d %d %.6f\n", kv.first.kind, kv.first.X, kv.first.Y, kv.first.part,
                 kv.first.bucket, kv.second.a, kv.second.b, kv.second.ms);
@@ -1087,14 +1090,17 @@ extern "C" int gtf_tune_save(const char *path)
 }
 
 // Merges a saved table; a file written on another device model is refused
-// (GTF_ERR_INVALID) and leaves the table unchanged.
+// (GTF_ERR_INVALID) and leaves the table unchanged.  Of an older version only
+// the entries of the dense products count: the blocks per SM of its Fock
+// launches would keep the present ones from their large blocks.
 extern "C" int gtf_tune_load(const char *path)
 {
     FILE *fp = fopen(path, "r");
     if (!fp) return GTF_ERR_IO;
     char magic[64], dev[256], here[256];
     int ver = 0;
-    if (fscanf(fp, "%63s %d %255s", magic, &ver, dev) != 3 || strcmp(magic, "gtfock_b200-tune") != 0 || ver != 1) {
+    if (fscanf(fp, "%63s %d %255s", magic, &ver, dev) != 3 || strcmp(magic, "gtfock_b200-tune") != 0 || ver < 1 ||
+        ver > GTF_TUNE_VERSION) {
         fclose(fp);
         return GTF_ERR_INVALID;
     }
@@ -1108,7 +1114,7 @@ extern "C" int gtf_tune_load(const char *path)
     TuneVal v;
     int r;
     while ((r = fscanf(fp, "%d %d %d %d %d %d %d %lf", &k.kind, &k.X, &k.Y, &k.part, &k.bucket, &v.a, &v.b, &v.ms)) == 8)
-        rows.push_back({k, v});
+        if (ver == GTF_TUNE_VERSION || k.kind == 2) rows.push_back({k, v});
     const bool ok = (r == EOF);
     fclose(fp);
     if (!ok) return GTF_ERR_INVALID;

@@ -100,7 +100,7 @@ struct FockGrid {
     int nsm;
     int fp32;                       // evaluate the integrals in FP32 (digestion stays FP64)
     // launch shape (autotuned; 0 = default): persistent blocks per SM (capped
-    // by the occupancy limit) and, in batched launches, units of 32 quartets
+    // by the occupancy limit) and, in batched launches, units of 32 lanes
     // a warp claims at once
     int ctas_per_sm;
     int claim;
@@ -114,7 +114,7 @@ struct FockGrid {
 };
 
 // ---------------------------------------------------------------------------
-// the Fock kernel: persistent warps claim units of 32 quartets
+// the Fock kernel: persistent warps claim units of 32 lanes
 // ---------------------------------------------------------------------------
 // Ket components per slice: quartets with up to 64 Cartesian integrals are
 // done in one pass; larger ones are split so that a slice keeps at most

@@ -88,14 +88,15 @@ PFockStatus_t gtf_pfock_shard_work(PFock_t pfock, double *work);
 /* Launch-shape autotuning.  gtf_pfock_autotune times, for every class pair
  * and precision part of this engine's Fock build (on the density last put),
  * candidate shapes of the persistent kernels -- blocks per SM (the occupancy
- * limit, one less, half), and in batched launches also the quartets a warp
+ * limit, one less, half), and in batched launches also the lanes of work a warp
  * claims at once (32, 64, 128) -- and records the fastest in a process-wide table keyed by (single / batch,
  * class pair, part, floor(log2(units of work))); later builds of any engine
  * or batch of that size use it.  gtf_batch_autotune does the same for a
  * batch's Fock launches and picks the tile shape of its batched dense
  * products (64x64, 32x32, 32x64, 128x64 output tiles).  The table is saved /
  * merged from a text file whose first line names the device model; a file
- * from another model is refused.  gtf_tune_entries writes rows of 8 ints
+ * from another model is refused, and of a file of older launch shapes only the
+ * entries of the dense products are taken.  gtf_tune_entries writes rows of 8 ints
  * (kind 0 single / 1 batch / 2 products, class X, class Y, part, size bucket,
  * blocks per SM or tile shape, claim, ms x 1000) and returns the count. */
 PFockStatus_t gtf_pfock_autotune(PFock_t pfock, int reps);

@@ -215,3 +215,31 @@ def test_admission_by_footprint():
     # the estimate grows with the basis and with incremental builds
     assert footprint_bytes(800) > footprint_bytes(400) > 0
     assert footprint_bytes(800, incremental=True) > footprint_bytes(800)
+
+
+def test_tuning_files_of_older_launch_shapes(tmp_path):
+    """A version 1 file holds Fock shapes measured on kernels with small blocks
+    (blocks per SM below the present occupancy limits, which would keep the
+    launches from their large blocks): only its dense-product entries count."""
+    L = gb.load()
+    gb.tune_clear()
+    L.gtf_tune_put(0, 1, 0, 0, 1e6, 3, 1, 0.5)
+    L.gtf_tune_put(1, 1, 0, 0, 1e6, 3, 2, 0.5)
+    L.gtf_tune_put(2, -1, -1, 0, 1e6, 1, 0, 0.5)
+    path = tmp_path / "tune.txt"
+    gb.tune_save(str(path))
+    gb.tune_clear()
+    gb.tune_load(str(path))
+    assert len(gb.tune_entries()) == 3
+    gb.tune_clear()
+    magic, version, rest = path.read_text().split(" ", 2)
+    assert version == "2"
+    path.write_text(" ".join([magic, "1", rest]))
+    gb.tune_load(str(path))
+    entries = gb.tune_entries()
+    assert [e["kind"] for e in entries] == ["products"]
+    gb.tune_clear()
+    path.write_text(" ".join([magic, "3", rest]))
+    with pytest.raises(gb.GtfError):
+        gb.tune_load(str(path))
+    assert gb.tune_entries() == []
