@@ -73,7 +73,7 @@ static const int k_cls_la[NCLS] = {0, 1, 1, 2, 2, 2};
 static const int k_cls_lb[NCLS] = {0, 0, 1, 0, 1, 2};
 
 struct UnitTask;
-#define UNIT_TOTALS 5   // totals per task (k_unit_totals)
+#define UNIT_TOTALS 8   // totals per task (k_unit_totals)
 
 static inline double __longlong_as_double_host(unsigned long long b)
 {
@@ -102,6 +102,9 @@ struct ClassPairTask {
     long long nunits, nunits32;  // units of the FP64 and the FP32 launch
     int split_lt;                // lane split of long quartets (gtf_lane_split)
     long long nunits_bound;      // bound on either launch's units under any thresholds >= tol2
+    // the same three with a quartet counted once, however many lanes share it:
+    // bras times 32 quartets, the size of the work to be shared out
+    long long nqunits, nqunits32, nqunits_bound;
     double flops, nprimq;        // Rys-model FLOPs and primitive quartets (before primitive screening)
     double nquart, nquart32;     // quartets in all, of which evaluated in FP32
     int *d_nket;                 // [nbra][GTF_NBKT] kets per (bra, segment)
@@ -1328,37 +1331,40 @@ static int shard_bounds(gtf_fock_dev *f, int c, const std::vector<int> &nk, cons
 
 // Totals of every task's (bra, segment) ket counts (task blockIdx.y): quartets,
 // FP32 quartets, the bound on a launch's units (sum over bras of the units of
-// all non-empty segments) and the units of the FP64 and the FP32 launch.
+// all non-empty segments), the units of 32 quartets of that bound and of the
+// FP64 and FP32 launches, and the units (32 lanes) of these launches.
 // 64-bit integer sums: exact whatever the order.
 __global__ void k_unit_totals(const UnitTask *__restrict__ tasks, unsigned long long *__restrict__ out)
 {
     const UnitTask &t = tasks[blockIdx.y];
     out += UNIT_TOTALS * blockIdx.y;
-    unsigned long long q = 0, q32 = 0, bound = 0;
+    unsigned long long v[6] = {0, 0, 0, 0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < t.nbra; i += gridDim.x * blockDim.x) {
-        const long long all = (long long)t.cum64[i * GTF_CUM + GTF_NBKT] + t.cum32[i * GTF_CUM + GTF_NBKT];
+        const long long lanes = (long long)t.cum64[i * GTF_CUM + GTF_NBKT] + t.cum32[i * GTF_CUM + GTF_NBKT];
+        long long all = 0, head = 0;
 #pragma unroll
         for (int b = 0; b < GTF_NBKT; b++) {
             const int k = i * GTF_NBKT + b;
-            q += (unsigned long long)t.nket[k];
-            q32 += (unsigned long long)(t.nket[k] - t.n64[k]);
+            v[0] += (unsigned long long)t.nket[k];
+            v[1] += (unsigned long long)(t.nket[k] - t.n64[k]);
+            if (b == 0) continue;   // no units
+            all += t.nket[k];
+            head += t.n64[k];
         }
-        bound += (unsigned long long)((all + 31) / 32);
+        v[2] += (unsigned long long)((lanes + 31) / 32);
+        v[3] += (unsigned long long)((all + 31) / 32);
+        v[4] += (unsigned long long)((head + 31) / 32);
+        v[5] += (unsigned long long)((all - head + 31) / 32);
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        q += __shfl_down_sync(GTF_FULL_MASK, q, o);
-        q32 += __shfl_down_sync(GTF_FULL_MASK, q32, o);
-        bound += __shfl_down_sync(GTF_FULL_MASK, bound, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(out, q);
-        atomicAdd(out + 1, q32);
-        atomicAdd(out + 2, bound);
+    for (int k = 0; k < 6; k++) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if ((threadIdx.x & 31) == 0) atomicAdd(out + k, v[k]);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        out[3] = (unsigned long long)t.up64[t.nbra];
-        out[4] = (unsigned long long)t.up32[t.nbra];
+        out[6] = (unsigned long long)t.up64[t.nbra];
+        out[7] = (unsigned long long)t.up32[t.nbra];
     }
 }
 
@@ -1378,6 +1384,7 @@ static int build_units(gtf_fock_dev *f)
     for (int c = 0; c < NCLSPAIR; c++) {
         ClassPairTask &t = f->tasks[c];
         t.nunits = t.nunits32 = 0;
+        t.nqunits = t.nqunits32 = 0;
         t.nquart = t.nquart32 = 0.0;
     }
     f->lists_dyn = 0;
@@ -1414,8 +1421,11 @@ static int build_units(gtf_fock_dev *f)
         // thresholds at or above tol2 select a subset of these kets, in one
         // launch or split between two (one more unit per bra at most)
         t.nunits_bound = (long long)q[2] + t.nbra;
-        t.nunits = (long long)q[3];
-        t.nunits32 = (long long)q[4];
+        t.nqunits_bound = (long long)q[3] + t.nbra;
+        t.nqunits = (long long)q[4];
+        t.nqunits32 = (long long)q[5];
+        t.nunits = (long long)q[6];
+        t.nunits32 = (long long)q[7];
         q += UNIT_TOTALS;
     }
     // the units of this engine's shard (all of them when not sharded)
@@ -2848,7 +2858,11 @@ struct gtf_fock_batch {
     SideLease held;   // side streams of a build under capture
 };
 
-// A molecule whose units in one launch reach this many (32 quartets each)
+// The rules below count units of 32 quartets, whatever lanes a quartet is
+// dealt out to (a small molecule's deep contractions take up to 32 lanes each,
+// and do not fill the GPU).
+//
+// A molecule whose units in one launch reach this many
 // fills the GPU by itself for ~70 rounds of its resident warps; it then runs
 // with the single-molecule kernel, which keeps its descriptor in the kernel
 // parameters (the batched kernel reads it from memory and holds the molecule
@@ -2992,7 +3006,7 @@ extern "C" int gtf_fock_batch_create(gtf_fock_dev_t *const *engines, int M, void
     std::vector<char> big(M, 0);
     for (int m = 0; m < M && !solo_env; m++) {
         long long tot = 0;
-        for (int c = 0; c < NCLSPAIR; c++) tot += engines[m]->tasks[c].nunits + engines[m]->tasks[c].nunits32;
+        for (int c = 0; c < NCLSPAIR; c++) tot += engines[m]->tasks[c].nqunits + engines[m]->tasks[c].nqunits32;
         big[m] = tot >= GTF_SOLO_MOL_UNITS;
     }
     // (incremental batches) the members' unit totals, per batched launch
@@ -3011,12 +3025,13 @@ extern "C" int gtf_fock_batch_create(gtf_fock_dev_t *const *engines, int M, void
                 // incremental: every part that can have work, sized by its bound
                 const long long nu = b->dyn ? ((p == 0 || f->prec == GTF_PREC_MIXED) ? t.nunits_bound : 0)
                                             : (p ? t.nunits32 : t.nunits);
+                const long long nqu = b->dyn ? t.nqunits_bound : p ? t.nqunits32 : t.nqunits;
                 if (nu == 0 || t.nbra == 0 || t.nketcls == 0) continue;
                 const bool need_tr = f->pure && f->nbf_cart != f->nbf;
                 FockLaunch a;
                 fill_launch(f, c, p, need_tr ? f->d_Dc : (b->dyn ? f->d_Dd : f->d_D), f->d_Fj, f->d_Fk, a);
                 const long long *tot = (p ? t.d_unit_prefix32 : t.d_unit_prefix) + t.nbra;
-                if (M > 1 && (nu >= solo_min || (big[m] && nu >= GTF_SOLO_MIN_UNITS))) {
+                if (M > 1 && (nqu >= solo_min || (big[m] && nqu >= GTF_SOLO_MIN_UNITS))) {
                     b->solo[c][p].push_back(a);
                     b->solo_units[c][p].push_back(nu);
                     b->solo_tot[c][p].push_back(tot);

@@ -147,6 +147,35 @@ def test_solo_launches_in_a_batch(tmp_path, monkeypatch):
     b.close()
 
 
+def test_solo_rule_counts_quartets(tmp_path, monkeypatch):
+    """A small molecule whose deep contractions are dealt out to many lanes each
+    has few quartets: it stays in the batched launches.  A class pair of Q
+    quartets over B bra pairs has at most Q / 32 + B units of 32 quartets;
+    with the threshold just above the largest of these, a step launches what
+    it does without one."""
+    xyz = mol.write_xyz(mol.alkane(2), str(tmp_path / "m.xyz"))
+    gbs = mol.basis_file("cc-pvdz")
+    basis = gb.BasisSet(gbs, xyz)
+    pf = gb.PFock(basis, tolscr=1e-10)
+    pf.compute_fock(np.eye(basis.nbf) * 0.3)
+    # 18 s, 10 p and 2 d shells: at most 18 x 10 pairs of one kind
+    most = int(max(q for _, _, _, q in pf.class_stats()) / 32) + 181
+    pf.close()
+    launches = []
+    for env in (None, str(most)):
+        if env:
+            monkeypatch.setenv("GTFOCK_SOLO_UNITS", env)
+        b = gb.Batch(4)
+        for _ in range(4):
+            b.add(gbs, xyz, max_iters=4, etol=0.0)
+        b.step()
+        n0 = gb.launch_count()
+        b.step()
+        launches.append(gb.launch_count() - n0)
+        b.close()
+    assert launches[0] == launches[1]
+
+
 def test_prepare_attach_while_stepping(tmp_path):
     """gtf_batch_prepare on one thread while the batch steps on another, then
     gtf_batch_attach between steps: the attached jobs give the oracle's
