@@ -1,6 +1,6 @@
 // purif.cu -- canonical density purification and Pulay DIIS on one GPU
 // (pscf/purif.c:257-641; the 3-D pdgemm of pscf/pdgemm.c becomes one product:
-// k_sym_abt for the symmetric ones, cuBLAS DGEMM for the others).
+// k_abt for D D^T and D D^2, cuBLAS DGEMM for the others).
 //
 // Purification (pscf/purif.c:301-476): Gershgorin bounds and tr F give the
 // initial D; each iteration forms D2 = D D^T and D3 = D D2, reduces
@@ -81,8 +81,8 @@ static int gemm_abt(gtf_purif_dev *p, const double *A, const double *B, double *
 }
 
 // ---------------------------------------------------------------------------
-// C = A B^T for products that are symmetric (D D and D D^2 of a symmetric D):
-// the tiles on and below the diagonal, mirrored.  Row-major n x n.
+// C = A B^T, row-major n x n.  SYM: for products that are symmetric (D D^T;
+// D D^2 of a symmetric D), the tiles on and below the diagonal, mirrored.
 //
 // One block per 32 x 32 tile; its four warps share the K loop (each takes 8 of
 // a slab's 32) and hold the whole tile in FP64 tensor-core accumulators
@@ -100,15 +100,28 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool o
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(ok ? 8 : 0) : "memory");
 }
 
-__global__ void __launch_bounds__(128) k_sym_abt(const double *__restrict__ A, const double *__restrict__ B,
-                                                 double *__restrict__ C, int n)
+// tile (ti, tj), tj <= ti, of the linear index ti (ti + 1) / 2 + tj
+__device__ __forceinline__ void tri_tile(int x, int &ti, int &tj)
+{
+    ti = (int)((sqrtf(8.0f * (float)x + 1.0f) - 1.0f) * 0.5f);
+    while (ti * (ti + 1) / 2 > x) ti--;
+    while ((ti + 1) * (ti + 2) / 2 <= x) ti++;
+    tj = x - ti * (ti + 1) / 2;
+}
+
+template <bool SYM>
+__global__ void __launch_bounds__(128) k_abt(const double *__restrict__ A, const double *__restrict__ B,
+                                             double *__restrict__ C, int n)
 {
     __shared__ __align__(16) double buf[2][2][ST_TILE * ST_LD];   // [stage][A or B]
-    // tile (ti, tj), tj <= ti, of the linear index ti (ti + 1) / 2 + tj
-    int ti = (int)((sqrtf(8.0f * (float)blockIdx.x + 1.0f) - 1.0f) * 0.5f);
-    while (ti * (ti + 1) / 2 > (int)blockIdx.x) ti--;
-    while ((ti + 1) * (ti + 2) / 2 <= (int)blockIdx.x) ti++;
-    const int tj = (int)blockIdx.x - ti * (ti + 1) / 2;
+    int ti, tj;
+    if constexpr (SYM) {
+        tri_tile((int)blockIdx.x, ti, tj);
+    } else {
+        const int nt = (n + ST_TILE - 1) / ST_TILE;
+        ti = (int)blockIdx.x / nt;
+        tj = (int)blockIdx.x - ti * nt;
+    }
     const int r0 = ti * ST_TILE, c0 = tj * ST_TILE;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     auto load = [&](int stage, int k0) {
@@ -171,8 +184,9 @@ __global__ void __launch_bounds__(128) k_sym_abt(const double *__restrict__ A, c
         const int r = e / ST_TILE, c = e % ST_TILE;
         double *p = part + r * 33 + c;
         p[0] = (p[0] + p[ST_TILE * 33]) + (p[2 * ST_TILE * 33] + p[3 * ST_TILE * 33]);
-        if (r0 + r < n && c0 + c <= r0 + r) C[(size_t)(r0 + r) * n + c0 + c] = p[0];
+        if (r0 + r < n && (SYM ? c0 + c <= r0 + r : c0 + c < n)) C[(size_t)(r0 + r) * n + c0 + c] = p[0];
     }
+    if constexpr (!SYM) return;
     __syncthreads();
     for (int e = threadIdx.x; e < ST_TILE * ST_TILE; e += 128) {
         const int c = e / ST_TILE, r = e % ST_TILE;
@@ -183,10 +197,44 @@ __global__ void __launch_bounds__(128) k_sym_abt(const double *__restrict__ A, c
 static int sym_abt(gtf_purif_dev *p, const double *A, const double *B, double *C)
 {
     const int nt = (p->n + ST_TILE - 1) / ST_TILE;
-    k_sym_abt<<<nt * (nt + 1) / 2, 128, 0, p->st>>>(A, B, C, p->n);
+    k_abt<true><<<nt * (nt + 1) / 2, 128, 0, p->st>>>(A, B, C, p->n);
     CKP(cudaGetLastError());
     gtf_note_launches(1);
     return GTF_OK;
+}
+
+static int full_abt(gtf_purif_dev_t *p, const double *A, const double *B, double *C)
+{
+    const int nt = (p->n + ST_TILE - 1) / ST_TILE;
+    k_abt<false><<<nt * nt, 128, 0, p->st>>>(A, B, C, p->n);
+    CKP(cudaGetLastError());
+    gtf_note_launches(1);
+    return GTF_OK;
+}
+
+// Largest |F - F^T|, as the bits of a double, into scal[12] (zeroed before)
+__global__ void __launch_bounds__(256) k_asymmetry(const double *__restrict__ F, int n, double *__restrict__ scal)
+{
+    __shared__ double t[ST_TILE][ST_TILE + 1];
+    int ti, tj;
+    tri_tile((int)blockIdx.x, ti, tj);
+    const int r0 = ti * ST_TILE, c0 = tj * ST_TILE, x = threadIdx.x % ST_TILE;
+    for (int y = threadIdx.x / ST_TILE; y < ST_TILE; y += 256 / ST_TILE)
+        if (r0 + y < n && c0 + x < n) t[y][x] = F[(size_t)(r0 + y) * n + c0 + x];
+    __syncthreads();
+    unsigned long long m = 0;
+    for (int y = threadIdx.x / ST_TILE; y < ST_TILE; y += 256 / ST_TILE)
+        if (c0 + y < n && r0 + x < n) {
+            const double d = fabs(F[(size_t)(c0 + y) * n + r0 + x] - t[x][y]);
+            const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+            m = b > m ? b : m;
+        }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long b = __shfl_xor_sync(0xffffffffu, m, o);
+        m = b > m ? b : m;
+    }
+    if ((threadIdx.x & 31) == 0 && m != 0) atomicMax((unsigned long long *)(scal + 12), m);
 }
 
 // sums over the 32 lanes, the same total in every lane
@@ -262,6 +310,9 @@ __global__ void k_purif_init(const double *__restrict__ part, int nblk, int n, i
     scal[3] = hmax;
     scal[4] = mu_bar;
     scal[5] = lambda;
+    // scal[13]: F is not symmetric but for rounding (1e-11 of its Gershgorin
+    // bound; X F X leaves 1e-14 to 1e-12), so D D^2 is not symmetric either
+    scal[13] = scal[12] <= 1e-11 * fmax(fabs(hmin), fabs(hmax)) ? 0.0 : 1.0;
 }
 
 __global__ void k_purif_d0(const double *__restrict__ F, double *__restrict__ D, int n, const double *scal)
@@ -570,11 +621,17 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
     cudaStream_t st = p->st;
     CKP(cudaEventRecord(p->e0, st));
     const int gb = (n + GERSH_COLS - 1) / GERSH_COLS;
+    const int nt = (n + ST_TILE - 1) / ST_TILE;
+    CKP(cudaMemsetAsync(p->scal + 12, 0, sizeof(double), st));
+    k_asymmetry<<<nt * (nt + 1) / 2, 256, 0, st>>>(F_dev, n, p->scal);
     k_gersh<<<gb, RED_THREADS, 0, st>>>(F_dev, n, p->part);
     k_purif_init<<<1, 32, 0, st>>>(p->part, gb, n, p->nocc, p->scal);
     k_purif_d0<<<ge, 256, 0, st>>>(F_dev, p->D, n, p->scal);
     CKP(cudaGetLastError());
-    gtf_note_launches(3);
+    gtf_note_launches(4);
+    CKP(cudaMemcpyAsync(p->h_scal + 13, p->scal + 13, sizeof(double), cudaMemcpyDeviceToHost, st));
+    CKP(cudaStreamSynchronize(st));
+    bool symmetric = p->h_scal[13] == 0.0;
     int it;
     double err = 0.0;
     // split-BF16 phase: tensor-core products until the error stops falling
@@ -596,6 +653,7 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
             CKP(cudaMemcpyAsync(p->h_scal + 6, p->scal + 6, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
             CKP(cudaStreamSynchronize(st));
             p->it_bf16++;
+            symmetric = true;
             const double e = p->h_scal[6];
             // hand over to FP64 once the error is small or stops falling
             // (BF16 rounding floor)
@@ -616,7 +674,7 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
     for (it = 0; it < PUR_MAX_ITERS && !stopped;) {
         for (int k = 0; k < PURIF_CHECK && it < PUR_MAX_ITERS; k++, it++) {
             if (sym_abt(p, p->D, p->D, p->D2)) return GTF_ERR_CUDA;
-            if (sym_abt(p, p->D, p->D2, p->D3)) return GTF_ERR_CUDA;
+            if (symmetric ? sym_abt(p, p->D, p->D2, p->D3) : full_abt(p, p->D, p->D2, p->D3)) return GTF_ERR_CUDA;
             k_purif_stats<<<RED_BLOCKS, RED_THREADS, 0, st>>>(p->D, p->D2, p->D3, n, p->part);
             k_purif_finish<<<1, 32, 0, st>>>(p->part, RED_BLOCKS, p->scal);
             k_purif_update<<<ge, 256, 0, st>>>(p->D, p->D2, p->D3, nn, p->scal);
