@@ -44,7 +44,9 @@ NMAX = 5            # roots needed for (dd|dd): L = 8 -> n = 5
 H64 = {1: 0.5, 2: 0.5, 3: 2.0, 4: 1.0, 5: 2.0}
 DEG64 = {1: 9, 2: 9, 3: 13, 4: 11, 5: 13}
 TMAX = {1: 40.0, 2: 48.0, 3: 56.0, 4: 62.0, 5: 70.0}
-# single-precision table for the mixed-precision kernels
+# single-precision table for the mixed-precision kernels: the classes of
+# fewer roots than NMIN32 use the Boys functions
+NMIN32 = 3
 H32 = 2.0
 DEG32 = 7
 # Boys functions: interval width, range, degrees of F_m and of (exp(-s) - 1) / s
@@ -139,10 +141,10 @@ def fit_boys(args):
                              HB, deg) + [mp.exp(-mid)]
 
 
-def build_table(h, deg, pool):
+def build_table(h, deg, pool, nmin=1):
     """h, deg: per root count (dict) or one value for all"""
     tables = {}
-    for n in range(1, NMAX + 1):
+    for n in range(nmin, NMAX + 1):
         hn = h[n] if isinstance(h, dict) else h
         dn = deg[n] if isinstance(deg, dict) else deg
         nint = int(round(TMAX[n] / hn))
@@ -163,7 +165,7 @@ def main(out_path=None):
                                 "csrc", "cuda", "rys_table.h")
     with mproc.get_context("spawn").Pool(os.cpu_count()) as pool:
         t64 = build_table(H64, DEG64, pool)
-        t32 = build_table(H32, DEG32, pool)
+        t32 = build_table(H32, DEG32, pool, NMIN32)
         nb = int(round(TB / HB))
         boys = {p: [pool.map(fit_boys, [(m, k, DEGB[p]) for k in range(nb)]) for m in range(BMAX + 1)]
                 for p in (64, 32)}
@@ -175,7 +177,7 @@ def main(out_path=None):
     w(" * in s = T - (T0 + H_n/2) for u_1..u_n then w_1..w_n, stored")
     w(" * [interval][coef][func]; above RYS_TMAX[n] the Hermite large-T form")
     w(" * u = x^2/T, w = W/sqrt(T) applies.  The FP32 table uses RYS32_H and")
-    w(" * RYS32_DEG for every n.  BOYS_TABLE, BOYS32_TABLE: see the generator. */")
+    w(" * RYS32_DEG, n = %d on.  BOYS_TABLE, BOYS32_TABLE: see the generator. */" % NMIN32)
     w("#pragma once")
     w("#ifndef RYS_QUAL")
     w("#define RYS_QUAL static")
@@ -208,7 +210,7 @@ def main(out_path=None):
     flat32 = []
     for n in range(1, NMAX + 1):
         offs32[n] = len(flat32)
-        flat32 += [iv[f][j] for iv in t32[n] for j in range(DEG32 + 1) for f in range(2 * n)]
+        flat32 += [iv[f][j] for iv in t32.get(n, []) for j in range(DEG32 + 1) for f in range(2 * n)]
     w("RYS_QUAL_SMALL const int RYS32_OFF[RYS_NMAX + 1] = {0, %s};" %
       ", ".join(str(offs32[n]) for n in range(1, NMAX + 1)))
     w("#define RYS32_OFF_LIST 0, %s" % ", ".join(str(offs32[n]) for n in range(1, NMAX + 1)))

@@ -1,7 +1,7 @@
 // Rounding errors of the integral building blocks, compiled for the host,
 // against 113-bit references.
 //   eri <class 0..11> <quartets>: one line "LA LB LC LD e64_rys e64_low
-//     e32_rys e32_low", geometric means over random contracted quartets of the
+//     e32_low", geometric means over random contracted quartets of the
 //     error relative to the quartet's largest integral, of the Rys form and of
 //     the form of eri_low.cuh (the reference: McMurchie-Davidson)
 //   boys: lines "m bits below above", largest error of F_m, m <= 4, in units of
@@ -177,7 +177,7 @@ static void eri_class(int n)
 {
     constexpr int NQ = ncart(LA) * ncart(LB) * ncart(LC) * ncart(LD), NCD = ncart(LC) * ncart(LD);
     constexpr int LT = LA + LB + LC + LD, NR = LT / 2 + 1;
-    double lg[4] = {0, 0, 0, 0};
+    double lg[3] = {0, 0, 0};
     for (int it = 0; it < n;) {
         // half of the quartets within 4 bohr a side, half up to 12 apart; some share centres
         double c[4][3];
@@ -210,20 +210,17 @@ static void eri_class(int n)
         const PPRec src{r64.data()};
         const PPRec32 src32{r32.data()};
         double o[2][NQ] = {};
-        float q[2][NQ] = {};
+        float q[NQ] = {};
         eri_accumulate_cd<LA, LB, LC, LD, 0, NCD, false, false, false>(src, pb, src, pk, o[0], RysTab<double>::ptr(NR));
         eri_accumulate_cd<LA, LB, LC, LD, 0, NCD, false, false, true>(src, pb, src, pk, o[1], BoysTab<double>::ptr(LT));
-        eri_accumulate_cd32<LA, LB, LC, LD, 0, NCD, false, false, false>(src32, pb, pk, q[0], RysTab<float>::ptr(NR));
-        eri_accumulate_cd32<LA, LB, LC, LD, 0, NCD, false, false, true>(src32, pb, pk, q[1], BoysTab<float>::ptr(LT));
-        for (int f = 0; f < 2; f++) {
-            double e = 1e-17, e32 = 1e-10;
-            for (int k = 0; k < NQ; k++) {
-                e = std::max(e, (double)fabsq(o[f][k] - ref[k]) / mx);
-                e32 = std::max(e32, (double)fabsq(q[f][k] - ref[k]) / mx);
-            }
-            lg[f] += log(e);
-            lg[2 + f] += log(e32);
+        eri_accumulate_cd32<LA, LB, LC, LD, 0, NCD, false, false, true>(src32, pb, pk, q, BoysTab<float>::ptr(LT));
+        double e[3] = {1e-17, 1e-17, 1e-10};
+        for (int k = 0; k < NQ; k++) {
+            e[0] = std::max(e[0], (double)fabsq(o[0][k] - ref[k]) / mx);
+            e[1] = std::max(e[1], (double)fabsq(o[1][k] - ref[k]) / mx);
+            e[2] = std::max(e[2], (double)fabsq(q[k] - ref[k]) / mx);
         }
+        for (int f = 0; f < 3; f++) lg[f] += log(e[f]);
     }
     printf("%d %d %d %d", LA, LB, LC, LD);
     for (double v : lg) printf(" %.4e", exp(v / n));
