@@ -53,7 +53,7 @@ SERVED_TAU = 1e-9
 SERVED_COUNT = 32        # requests of the served stream in the default run
 # DRAM bytes (read + write) of all k_fock launches of one C54H18 build, from one
 # ncu capture (profiles/fock_c54h18_dram_traffic.md); the kernels are FP64 bound
-FOCK_BUILD_DRAM_BYTES = 648.2e6 + 84.9e6
+FOCK_BUILD_DRAM_BYTES = 548.0e6 + 0.3e6
 METRIC = "SCF solves/s (C54H18 cc-pVDZ, 10 iterations, FP64)"
 WORKLOAD = "C54H18 graphene flake / cc-pVDZ (846 bf), Schwarz 1e-10, 10 SCF iterations, FP64"
 
@@ -326,8 +326,9 @@ def run(args):
         tm = pf.timing()
         counts = pf.counts()
         eri_flops = tm["eri_flops"]
-        # the same model over the primitive quartets the kernels evaluate
-        # (after primitive screening at |K_ab K_cd| < 1e-17)
+        # the roofline counts the primitive quartets the kernels evaluate (after
+        # primitive screening at |K_ab K_cd| < 1e-15); the same model over all
+        # of them is reported beside it
         scr = pf.class_work_screened()
         eri_flops_scr = sum(w[0] for w in scr)
         primq_scr = sum(w[1] for w in scr)
@@ -349,7 +350,7 @@ def run(args):
         fp64_peak = gb.fp64_peak_gflops()
     value = world * args.steps / dt
     eri_s = statistics.median(eri_ms) * 1e-3
-    achieved = eri_flops / eri_s / 1e12
+    achieved = eri_flops_scr / eri_s / 1e12
     peak = fp64_peak / 1e3
     line = {
         "metric": METRIC, "value": value, "unit": "solves/s", "n_gpus": world,
@@ -371,14 +372,14 @@ def run(args):
                      "kernel": "k_fock<*> (all class pairs of one Fock build)",
                      "peak_source": "FP64 FMA probe kernel measured in this run "
                                     "(MEASURED_PEAKS.json has no FP64 figure)",
-                     "work": "Rys-model FLOPs per build %.4g, over every primitive quartet of every "
-                             "screened quartet (before primitive screening)" % eri_flops,
+                     "work": "Rys-model FLOPs per build %.4g, over the %.4g primitive quartets left by "
+                             "primitive screening (the light classes do less: Boys functions and "
+                             "recurrences)" % (eri_flops_scr, primq_scr),
                      "eri_ms_per_build": eri_s * 1e3,
-                     "after_primitive_screening": {
-                         "work_flops": eri_flops_scr, "primitive_quartets": primq_scr,
-                         "primitive_quartets_before": primq_all,
-                         "achieved": eri_flops_scr / eri_s / 1e12,
-                         "frac": eri_flops_scr / eri_s / 1e12 / peak}},
+                     "before_primitive_screening": {
+                         "work_flops": eri_flops, "primitive_quartets": primq_all,
+                         "achieved": eri_flops / eri_s / 1e12,
+                         "frac": eri_flops / eri_s / 1e12 / peak}},
         "clocks": clocks,
         "mixed_precision": {"value": world * args.steps / dt_mixed, "unit": "solves/s",
                             "fp32_cutoff": MIXED_CUTOFF,
@@ -386,8 +387,10 @@ def run(args):
                             "note": "FP32 ERIs for quartets with Schwarz bound below the cutoff; "
                                     "digestion and F accumulation FP64. The 10-iteration C54H18 SCF "
                                     "from the core-Hamiltonian guess is not converged and its iterates "
-                                    "differ by ~0.05 Ha between two FP64 runs (atomic summation "
-                                    "order), so dE_last_vs_fp64 measures that, not the FP32 error; "
+                                    "follow the rounding of the early, ill-conditioned steps: ~0.05 Ha "
+                                    "between two FP64 runs at worst, ~20 Ha with the split-BF16 "
+                                    "purification of this mode, so dE_last_vs_fp64 measures that, not the "
+                                    "FP32 error (1e-5 Ha with FP64 purification); "
                                     "converged energies agree within 1e-11 Ha (--workload precision)"},
     }
     if world == 1 and not args.quick:

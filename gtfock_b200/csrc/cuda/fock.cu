@@ -2115,7 +2115,8 @@ static int launch_class(const gtf_fock_dev *f, int c, const double *D, double *F
 // them over several streams.  A launch of a small molecule occupies a few SMs
 // for the latency of its longest lane, and up to 62 of them (124 in mixed
 // precision) in a row add up (ethane / cc-pVDZ 2.0 -> 0.47 ms, C12H26 8.9 ->
-// 7.7 ms).  Above, one launch fills the GPU: overlapping tails gained at most
+// 7.7 ms; 0.38 ms for ethane without events around the classes, whose times
+// are measured apart).  Above, one launch fills the GPU: overlapping tails gained at most
 // 0.5% on C54H18 / cc-pVDZ (13.4M units) and (H2O)64 / 6-31G (9.8M), and the
 // times per class pair would no longer add up.
 #define GTF_OVERLAP_UNITS 2000000LL

@@ -145,7 +145,10 @@ __host__ __device__ constexpr int fock_slice(int LA, int LB, int LC, int LD, int
 // 6.99 7.11 (of 10), (ps|ss) 21.8 21.2 21.1, (ps|ps) 14.9 15.1 15.5 (but
 // (H2O)64 5.92 5.78 5.97), (ds|ps) 14.6 14.2, (pp|ps) 15.6 13.2 13.9; the Rys
 // classes of 54 integrals lose 25-50% with 3 blocks in FP64 (spills) and gain
-// 3-5% in FP32.  No primitive record is loaded ahead: with this many warps a
+// 3-5% in FP32.  (Taken with the horizontal transfer in the light classes;
+// raising the second index directly added 1-19% to those that had it, the most
+// to (dp|ps), 12.5 -> 14.8 ms, which spills 112 bytes.)  No primitive record is
+// loaded ahead: with this many warps a
 // load's latency is hidden, and the registers of two records more cost
 // 6% of the build in spills.
 __host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD, int fp32)
@@ -157,13 +160,11 @@ __host__ __device__ constexpr int fock_min_blocks(int LA, int LB, int LC, int LD
     return nq <= (fp32 ? 54 : 36) ? 3 : 2;
 }
 
-//
 // A launch with many units per SM runs one block of fock_max_threads on each
-// (two, of at most 1024 threads), so that the SM holds one copy of the class's
-// table (up to 49 KB) and the rest
-// of its 228 KB caches the gathers of D and of the primitive records; small
-// launches spread blocks of FOCK_THREADS over the SMs.  The registers per
-// thread are the same.
+// (two, where that would be more than 1024 threads), so that the SM holds one
+// copy of the class's table (up to 49 KB) and the rest of its 228 KB caches the
+// gathers of D and of the primitive records; small launches spread blocks of
+// FOCK_THREADS over the SMs.  The registers per thread are the same.
 __host__ __device__ constexpr int fock_big_blocks(int LA, int LB, int LC, int LD, int fp32)
 {
     return FOCK_THREADS * fock_min_blocks(LA, LB, LC, LD, fp32) > 1024 ? 2 : 1;

@@ -310,9 +310,6 @@ __global__ void k_purif_init(const double *__restrict__ part, int nblk, int n, i
     scal[3] = hmax;
     scal[4] = mu_bar;
     scal[5] = lambda;
-    // scal[13]: F is not symmetric but for rounding (1e-11 of its Gershgorin
-    // bound; X F X leaves 1e-14 to 1e-12), so D D^2 is not symmetric either
-    scal[13] = scal[12] <= 1e-11 * fmax(fabs(hmin), fabs(hmax)) ? 0.0 : 1.0;
 }
 
 __global__ void k_purif_d0(const double *__restrict__ F, double *__restrict__ D, int n, const double *scal)
@@ -621,17 +618,11 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
     cudaStream_t st = p->st;
     CKP(cudaEventRecord(p->e0, st));
     const int gb = (n + GERSH_COLS - 1) / GERSH_COLS;
-    const int nt = (n + ST_TILE - 1) / ST_TILE;
-    CKP(cudaMemsetAsync(p->scal + 12, 0, sizeof(double), st));
-    k_asymmetry<<<nt * (nt + 1) / 2, 256, 0, st>>>(F_dev, n, p->scal);
     k_gersh<<<gb, RED_THREADS, 0, st>>>(F_dev, n, p->part);
     k_purif_init<<<1, 32, 0, st>>>(p->part, gb, n, p->nocc, p->scal);
     k_purif_d0<<<ge, 256, 0, st>>>(F_dev, p->D, n, p->scal);
     CKP(cudaGetLastError());
-    gtf_note_launches(4);
-    CKP(cudaMemcpyAsync(p->h_scal + 13, p->scal + 13, sizeof(double), cudaMemcpyDeviceToHost, st));
-    CKP(cudaStreamSynchronize(st));
-    bool symmetric = p->h_scal[13] == 0.0;
+    gtf_note_launches(3);
     int it;
     double err = 0.0;
     // split-BF16 phase: tensor-core products until the error stops falling
@@ -653,7 +644,6 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
             CKP(cudaMemcpyAsync(p->h_scal + 6, p->scal + 6, sizeof(double) * 2, cudaMemcpyDeviceToHost, st));
             CKP(cudaStreamSynchronize(st));
             p->it_bf16++;
-            symmetric = true;
             const double e = p->h_scal[6];
             // hand over to FP64 once the error is small or stops falling
             // (BF16 rounding floor)
@@ -666,9 +656,19 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
             }
         }
     }
-    // FP64 canonical steps (from the split-BF16 state in mode 1), PURIF_CHECK
-    // launched per host read of the device-side stop flag
-    CKP(cudaMemsetAsync(p->scal + 8, 0, sizeof(double) * 4, st));
+    // FP64 canonical steps (from the split-BF16 state in mode 1, which is
+    // symmetrised), PURIF_CHECK launched per host read of the device-side stop
+    // flag.  The first read also tells whether F was symmetric but for rounding
+    // (1e-11 of its Gershgorin bound; X F X leaves 1e-14 to 1e-12).  If not, D D^2
+    // is not symmetric either, and the loop starts again with it in full.
+    CKP(cudaMemsetAsync(p->scal + 8, 0, sizeof(double) * 5, st));
+    bool known = p->it_bf16 > 0, symmetric = true;
+    if (!known) {
+        const int nt = (n + ST_TILE - 1) / ST_TILE;
+        k_asymmetry<<<nt * (nt + 1) / 2, 256, 0, st>>>(F_dev, n, p->scal);
+        CKP(cudaGetLastError());
+        gtf_note_launches(1);
+    }
     int steps = 0;
     bool stopped = false;
     for (it = 0; it < PUR_MAX_ITERS && !stopped;) {
@@ -681,11 +681,23 @@ extern "C" int gtf_purif_run_dev(gtf_purif_dev_t *p, const double *F_dev, double
             CKP(cudaGetLastError());
             gtf_note_launches(3);
         }
-        CKP(cudaMemcpyAsync(p->h_scal + 6, p->scal + 6, sizeof(double) * 4, cudaMemcpyDeviceToHost, st));
+        CKP(cudaMemcpyAsync(p->h_scal + 2, p->scal + 2, sizeof(double) * 11, cudaMemcpyDeviceToHost, st));
         CKP(cudaStreamSynchronize(st));
         err = p->h_scal[6];
         steps = (int)p->h_scal[9];
         stopped = p->h_scal[8] != 0.0;
+        if (!known) {
+            known = true;
+            symmetric = p->h_scal[12] <= 1e-11 * fmax(fabs(p->h_scal[2]), fabs(p->h_scal[3]));   // false for a NaN
+            if (!symmetric) {
+                k_purif_d0<<<ge, 256, 0, st>>>(F_dev, p->D, n, p->scal);
+                CKP(cudaGetLastError());
+                gtf_note_launches(1);
+                CKP(cudaMemsetAsync(p->scal + 8, 0, sizeof(double) * 4, st));
+                it = 0;
+                stopped = false;
+            }
+        }
     }
     p->errnorm = err;
     // the counts of the reference's loop: steps run, and the index of the
